@@ -174,6 +174,69 @@ struct Contraction {
   }
 };
 
+// The nucleus heuristic's contraction (sample.rs:658-698) asks one question of the product
+// of multipliers, at iterate nucleus + 1: is its squared modulus below 1e-6? This keeps the
+// squared modulus alone, p 2^e with p in [2^-420, 2^420], from the squares of the factors'
+// moduli: one multiply and one range test an iteration in place of a complex product and
+// the range tests of its factors and parts.
+// Every factor and product rounds within 4 units, Contraction's within 5 (normwise,
+// squared), so the two differ by less than 9 u a step. small() answers outside a band of
+// 32 u (nucleus + 8) around 1e-6 and returns -1 inside it, or where the product was lost (a
+// zero or non-finite factor, or a count beyond e's range): the sample is then iterated
+// again from its start with Contraction itself (exact()).
+#ifndef FDK_CONTRACTION_AGAIN
+#define FDK_CONTRACTION_AGAIN false  // a test build answers -1 always
+#endif
+struct Magnitude {
+  double p;  // NaN: lost, or exact()
+  int32_t e;
+  __device__ __forceinline__ void reset(int32_t nucleus) {  // e counts up to 2 nucleus: 32 bits hold it below 2^29
+    p = nucleus < (1 << 29) ? 1.0 : __longlong_as_double(0x7ff8000000000000ll);
+    e = 0;
+  }
+  __device__ __forceinline__ void take_exact() {
+    p = __longlong_as_double(0x7ff8000000000000ll);
+    e = INT32_MIN;
+  }
+  __device__ __forceinline__ bool exact() const { return e == INT32_MIN; }
+  // times q 2^up, q = r^2 + i^2, where that is quick (p q in range means q >= 2^-840: nothing
+  // that counts has underflowed in it); false leaves the product as it was
+  __device__ __forceinline__ bool times(double q, int up) {
+    const double t = p * q;
+    const uint32_t hi = (uint32_t)__double2hiint(t);
+    const bool in = hi - ((1023u - 420u) << 20) < (840u << 20);
+    if (in) p = __hiloint2double((int)(hi + ((uint32_t)up << 20)), __double2loint(t));
+    return in;
+  }
+  static __device__ __forceinline__ int exponent(double a) { return (int)((uint32_t)__double2hiint(a) >> 20) - 1023; }
+  static __device__ __forceinline__ double mantissa(double a) {  // of a normal a > 0, in [1, 2)
+    return __hiloint2double((int)(((uint32_t)__double2hiint(a) & 0xfffffu) | 0x3ff00000u), __double2loint(a));
+  }
+  // the same for factors of any size
+  __device__ __forceinline__ void times_wide(double r, double i) {
+    const double a = rmax(fabs(r), fabs(i));
+    const int up = a < 0x1p-400 ? 600 : (a > 0x1p400 ? -600 : 0);
+    const double f = exp2i(up);
+    r = r * f;
+    i = i * f;
+    const double q = r * r + i * i;
+    if (a > 0.0 && isfinite(a) && p > 0.0) {
+      e += exponent(p) + exponent(q) - 2 * up;
+      p = mantissa(p) * mantissa(q);
+    } else {
+      p = __longlong_as_double(0x7ff8000000000000ll);
+    }
+  }
+  __device__ __forceinline__ int small(int32_t nucleus) const {
+    if (FDK_CONTRACTION_AGAIN || !(p > 0.0)) return -1;
+    const int64_t top = (int64_t)e + exponent(p);
+    if (top > 0) return 0;
+    if (top < -64) return 1;
+    const double v = mantissa(p) * exp2i(top), band = 32.0 * U * ((double)nucleus + 8.0);
+    return v < 1e-6 * (1.0 - band) ? 1 : (v > 1e-6 * (1.0 + band) ? 0 : -1);
+  }
+};
+
 // sample.rs:1094-1114 for two terms.
 static __device__ __noinline__ Cx3 sum2(Cx3 a, Cx3 b, int64_t zero_e) {
   bool have = false;

@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(128) perturb_noalloc_kernel(fdk::Params p, uns
   State<EXT> s;
   Result res;
   bool active = false, exhausted = false;
+  ExactProduct product;
   unsigned long long n_samples = 0, iters = 0;
   auto finish = [&](uint32_t idx, const Result &r) {
     put(p, idx, r);
@@ -98,9 +99,15 @@ __global__ void __launch_bounds__(128) perturb_noalloc_kernel(fdk::Params p, uns
       need = __ballot_sync(FULL, !active);
     }
     if (!__any_sync(FULL, active)) break;
-    if (active && step<EXT, D, false>(p, s, res)) {
-      finish(s.idx, res);
-      active = false;
+    if (active && step<EXT, D>(p, s, res, product)) {
+      if (res.kind == 3) {  // once more, for Contraction's own product
+        start_sample<EXT, D, false, false>(p, s, false, false);
+        s.ct.take_exact();
+        product.reset();
+      } else {
+        finish(s.idx, res);
+        active = false;
+      }
     }
   }
   for (int o = 16; o > 0; o >>= 1) {

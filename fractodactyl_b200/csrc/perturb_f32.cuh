@@ -476,6 +476,13 @@ __device__ __forceinline__ bool post_f32(const Params &p, const Entry32 *__restr
   return false;
 }
 
+// A lane's BLA block found but not yet applied.
+struct Waiting {
+  bool on;
+  int lv;
+  uint32_t at;
+};
+
 // One iteration of the precision form for the active lanes of a warp, with the block
 // deferral of warp_step.
 template <bool D, bool L>

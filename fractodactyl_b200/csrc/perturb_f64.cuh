@@ -13,6 +13,10 @@ namespace fdk {
 
 constexpr int MAX_LEVELS = 40;
 
+#if !defined(__CUDACC__) && !defined(__grid_constant__)
+#define __grid_constant__  // host builds of this header
+#endif
+
 // Resident 128-thread blocks per SM each kernel variant is compiled for (caps registers
 // at 65536 / (128 * blocks)): floatexp-tier variants (EXT) and ordinary-tier variants;
 // chosen by measurement (5 floatexp blocks at 96 registers: the 1920x1080 frame at a 1e-100
@@ -103,6 +107,7 @@ struct Params {
 };
 
 constexpr double SAFE = 1.0 + 8.0 * U;  // sample.rs:56
+constexpr uint32_t NO_GATE = 0xffffffffu;
 
 enum : uint32_t { F_DERIV = 1u, F_BLA = 2u, F_SHIFT = 4u };
 
@@ -112,22 +117,23 @@ struct State {
   double xr, xi, dr, di;
   double fr, fi;  // z = Z[m] + delta (carried between steps on the ordinary tier)
   double Zr, Zi;  // Z[m]
-  double r2a, r2b;  // radii^2 of the blocks of 2 and 4 steps starting at m (BLA kernels)
+  double r2a;     // radius^2 of the block of 2 steps starting at m, -1 where none starts (BLA kernels)
   double ar, ai;  // sample offset (mantissa on the extended tier)
   double dc_r, dc_i, scale, inverse;
   double sr, si, qr, qi, qstep;
-  double near;  // save_point(): the near-return bound of the save point (sr, si)
+  double near;  // save_point(): the near-return bound of the save point; infinite while a save is pending
   Multiplier mu;
-  Contraction ct;
+  Magnitude ct;
   double adc, shift;
   double e, ed, rc;  // B: error radii on z and dz/dc, the offset's own error (sample.rs:221-225)
   int32_t offset_exp, delta_exp;  // |h_e| <= 2^30 (checked by the route): deltas stay within 32 bits
   int64_t derivative_exp;
-  int32_t nucleus;               // < 2^31 - 1 (checked by the route)
+  uint32_t gate;  // the nucleus gate's iterate, nucleus + 1 < 2^31, or NO_GATE
   uint32_t n, chk, sn, hold, blocks, skipped;  // n < max_iter < 2^32; chk saturates at 2^32 - 1
   uint32_t lim;  // relimit()
   uint32_t m, idx;
   int returns;
+  bool on;  // the next operation is a BLA block (set by post)
   bool pending, predicted;
   bool replaying;  // T: re-walking a stripe window plainly (sample.rs:231-236) ...
   uint32_t limit;  // ... up to this iterate
@@ -256,32 +262,45 @@ struct StripeTrace {
 // A periodicity save point (sample.rs:488-491, 522-575): the point and the bound that a
 // later z's distance from it is compared with, fabs(sr) + fabs(si) scaled as each tier's
 // near-return test scales it. The reference evaluates the bound every iteration from the
-// same two values, so evaluating it once here gives the same double.
+// same two values, so evaluating it once here gives the same double. While a save is
+// pending every judged z is an event: the bound is infinite (sequence() takes near_bound).
+template <bool EXT>
+__device__ __forceinline__ double near_bound(const State<EXT> &s) {
+  const double size = fabs(s.sr) + fabs(s.si);
+  return EXT ? 1e-13 * size + 1e-300 : 1e-3 * size;
+}
+
 template <bool EXT>
 __device__ __forceinline__ void save_point(State<EXT> &s, double r, double i) {
   s.sr = r;
   s.si = i;
-  const double size = fabs(r) + fabs(i);
-  s.near = EXT ? 1e-13 * size + 1e-300 : 1e-3 * size;
+  s.near = near_bound(s);
+}
+
+template <bool EXT>
+__device__ __forceinline__ void await_save(State<EXT> &s) {  // the next judged iterate is saved
+  s.pending = true;
+  s.near = __longlong_as_double(0x7ff0000000000000ll);
 }
 
 // The iteration limit behind Bla::find's budget (sample.rs:246-263) with n left out:
 // min(max_iter, the next periodicity save point, nucleus + 1), kept in the state and
-// recomputed whenever one of its inputs (hold, sn, pending, chk, nucleus) changes, so an
+// recomputed whenever one of its inputs (hold, sn, pending, chk, gate) changes, so an
 // iteration only subtracts n. The reference's n == 0 case (a budget of 1) never reaches
 // the search: with a nucleus gate, m == 0 skips the BLA. lim <= max_iter < 2^32.
 template <bool EXT>
 __device__ __forceinline__ void relimit(const Params &p, State<EXT> &s) {
-  uint64_t cap = s.hold > 0 ? (uint64_t)s.sn + s.hold : (s.pending ? ~0ull : (uint64_t)s.chk);
-  uint64_t b = p.max_iter < cap ? p.max_iter : cap;
-  if (s.nucleus >= 0 && (uint64_t)s.nucleus + 1 < b) b = (uint64_t)s.nucleus + 1;
-  s.lim = (uint32_t)b;
+  uint32_t cap = s.chk;
+  if (!EXT) {
+    const uint32_t back = s.sn + s.hold;
+    cap = s.hold > 0 ? (back < s.sn ? 0xffffffffu : back) : (s.pending ? 0xffffffffu : s.chk);
+  }
+  s.lim = min(min(p.max_iter, cap), s.gate);
 }
 
-// Bla::find (bla.rs:234-249) at the top of an iteration: the level of the longest valid
-// block starting at m that fits the budget, or -1, with its index in that level in `at`.
-// The radii of the first two levels come with the orbit entry (r2a, r2b); those of the
-// next PRE levels are loaded together before the comparisons that would stop at them.
+// Bla::find (bla.rs:234-249): the longest valid block starting at m that fits the budget.
+// The radius of the first level comes with the orbit entry (r2a); block_starts tests it, and
+// block_level searches the others once the lane's turn to apply a block has come.
 template <bool EXT>
 __device__ __forceinline__ double block_d2(const State<EXT> &s) {
   return EXT ? (s.xr * s.xr + s.xi * s.xi) * s.scale * s.scale : s.xr * s.xr + s.xi * s.xi;
@@ -293,7 +312,7 @@ __device__ __forceinline__ double block_d2(const State<EXT> &s) {
 template <bool EXT>
 __device__ __forceinline__ bool block_starts(const State<EXT> &s) {
   const uint32_t budget = s.lim > s.n ? s.lim - s.n : 0u;
-  return (s.nucleus < 0 || s.m != 0) & (budget >= 2) & (block_d2(s) < s.r2a);
+  return (s.gate == NO_GATE || s.m != 0) & (budget >= 2) & (block_d2(s) < s.r2a);
 }
 
 // The rest of Bla::find once block_starts holds: the level of the longest valid block.
@@ -303,7 +322,7 @@ __device__ __forceinline__ int block_level(const Params &p, const State<EXT> &s,
   const double d2 = block_d2(s);
   const uint32_t k = s.m - 1u;     // m = 0 wraps: odd, no block
   at = k >> 1;
-  if (budget < 4 || !(d2 < s.r2b)) return 0;
+  if (budget < 4 || !(d2 < __ldg(p.fused + 2 * s.m + 1).y)) return 0;
   at = k >> 2;
   const uint32_t tz = k == 0 ? 32u : (uint32_t)(__ffs((int)k) - 1);
   const uint32_t top = tz < p.bla_levels ? tz : p.bla_levels;
@@ -336,18 +355,74 @@ __device__ __forceinline__ int block_level(const Params &p, const State<EXT> &s,
   return lv;
 }
 
+// Contraction's own product of a lane's sample, kept in memory: only a sample iterated again
+// for it (Magnitude) reads or writes it.
+struct ExactProduct {
+  volatile double re, im;
+  volatile int64_t exp;
+  volatile bool started;
+  __device__ __forceinline__ void reset() {
+    re = 0.0;
+    im = 0.0;
+    exp = 0;
+    started = false;
+  }
+  __device__ __forceinline__ Contraction get() const { return Contraction{re, im, exp, started}; }
+  __device__ __forceinline__ void multiply(double r, double i) {
+    Contraction c = get();
+    c.multiply(r, i);
+    re = c.re;
+    im = c.im;
+    exp = c.exp;
+    started = c.started;
+  }
+};
+
+// A factor (r, i) that Magnitude::times did not take: of any size, or for Contraction itself
+// where the sample is iterated again for it.
 template <bool EXT>
-__device__ __forceinline__ int find_block(const Params &p, const State<EXT> &s, uint32_t &at) {
-  return block_starts(s) ? block_level(p, s, at) : -1;
+__device__ __forceinline__ void contraction_wide(State<EXT> &s, ExactProduct &product, double r, double i) {
+  if (s.gate == NO_GATE)
+    s.ct.reset(0);  // no longer asked for
+  else if (s.ct.exact())
+    product.multiply(r, i);
+  else
+    s.ct.times_wide(r, i);
+}
+
+// The orbit entry at m: Z_m, and with BLA the squared radius of the first-level block there,
+// in one 32-byte load (its fourth value, the second level's radius, is read by block_level).
+struct Entry {
+  double zr, zi, r2a;
+};
+
+template <bool L>
+__device__ __forceinline__ Entry load_entry(const Params &p, uint32_t m) {
+  if (L) {
+#if defined(__CUDA_ARCH__)
+    Entry e;
+    double r2b;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(e.zr), "=d"(e.zi), "=d"(e.r2a), "=d"(r2b)
+        : "l"(p.fused + 2 * m));
+    return e;
+#else
+    const double2 Z = __ldg(p.fused + 2 * m), R = __ldg(p.fused + 2 * m + 1);
+    return Entry{Z.x, Z.y, R.x};
+#endif
+  }
+  const double2 Z = __ldg(p.orbit + m);
+  return Entry{Z.x, Z.y, -1.0};
 }
 
 // A BLA block application (sample.rs:264-315): delta' = A delta + B dc, dz' = A dz + B.
 template <bool EXT, bool D>
-__device__ __forceinline__ void apply_block(const Params &p, State<EXT> &s, int lv, uint32_t at) {
+__device__ __forceinline__ void apply_block(const Params &p, State<EXT> &s, int lv, uint32_t at,
+                                            ExactProduct &product) {
   const uint32_t b = p.bla_off[lv] + at;
   const double2 A = __ldg(p.bla_coef + 2 * b), B = __ldg(p.bla_coef + 2 * b + 1);
   const uint32_t len = 2u << lv;
-  if (s.nucleus >= 0 && s.n >= 1) s.ct.multiply(A.x, A.y);
+  if (__builtin_expect(!s.ct.times(A.x * A.x + A.y * A.y, 0), 0)) contraction_wide(s, product, A.x, A.y);
   if (!EXT && s.hold > 0) s.mu.multiply(A.x, A.y);
   if (EXT) {
     normalise(s.xr, s.xi, s.delta_exp, 0);
@@ -394,7 +469,6 @@ __device__ __forceinline__ void apply_block(const Params &p, State<EXT> &s, int 
 template <bool EXT, bool D, bool B = false>
 __device__ __forceinline__ void plain_update(State<EXT> &s, const double *__restrict__ q = nullptr) {
   const double fr = s.fr, fi = s.fi;
-  if (s.nucleus >= 0 && s.n >= 1) s.ct.multiply(2.0 * fr, 2.0 * fi);
   if (!EXT && s.hold > 0) s.mu.multiply(2.0 * fr, 2.0 * fi);
   if (B) {  // sample.rs:338-350: the radii through this step, from the state before it
     const double qm = __ldg(q + s.m);
@@ -412,12 +486,6 @@ __device__ __forceinline__ void plain_update(State<EXT> &s, const double *__rest
     double t = 2.0 * (fr * s.dr - fi * s.di) + s.inverse;
     s.di = 2.0 * (fr * s.di + fi * s.dr);
     s.dr = t;
-    if (EXT && rmax(fabs(s.dr), fabs(s.di)) > HI) {
-      s.dr = s.dr * LO;
-      s.di = s.di * LO;
-      s.derivative_exp += 32;
-      s.inverse = exp2i(-s.derivative_exp);
-    }
   }
   const double wr = s.xr, wi = s.xi, zr = s.Zr, zi = s.Zi;
   if (EXT) {  // number.rs:109-124
@@ -431,109 +499,15 @@ __device__ __forceinline__ void plain_update(State<EXT> &s, const double *__rest
   s.n += 1;
 }
 
-// The rest of the iteration after the update (sample.rs:381-575): the next orbit point,
-// bailout, nucleus gate, rebase, rescaling and periodicity. Zn/Rn hold the prefetched
-// entry m + 1 of the iteration's start, right after a plain step; after a block (took)
-// the entry at the new m is loaded here. Returns true when the sample has an outcome.
-// T: the Stripe recorder tr records the iterate, and an escape whose window misses
-// iterates replays them from a kept block start (sample.rs:369-403).
-template <bool EXT, bool D, bool L, bool B = false, bool T = false>
-__device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res, bool took, double2 Zn,
-                                     double2 Rn, StripeTrace *tr = nullptr) {
-  double2 Z = Zn;
-  if (L) {
-    if (took) {  // a block moved m by its length
-      Z = __ldg(p.fused + 2 * s.m);
-      Rn = __ldg(p.fused + 2 * s.m + 1);
-    }
-    s.r2a = Rn.x;
-    s.r2b = Rn.y;
-  }
-  s.Zr = Z.x;
-  s.Zi = Z.y;
-  double pr = EXT ? s.scale * s.xr : s.xr, pi = EXT ? s.scale * s.xi : s.xi;
-  double fr = Z.x + pr, fi = Z.y + pi;
-  double f2 = fr * fr + fi * fi;
-  if (T) tr->record(s.n, fr, fi);
+// The full sequence after an update (sample.rs:381-575) for iterations in which some event
+// may have happened: bailout, nucleus gate, rebase, rescaling, periodicity. z = (fr, fi) with
+// |z|^2 = f2 at the entry Z of the new m, the physical delta (pr, pi). Returns true when the
+// sample has an outcome (kind 3: none yet, to be iterated again for Contraction's product).
+template <bool EXT, bool D, bool L, bool B, bool T>
+__device__ __forceinline__ bool sequence(const Params &p, State<EXT> &s, Result &res, double2 Z, double pr, double pi,
+                                         double fr, double fi, double f2, ExactProduct &product,
+                                         StripeTrace *tr) {
   const bool replaying = T && s.replaying;  // no nucleus gate or periodicity while replaying
-  {
-    // The common iterations leave through a short path: no escape, nucleus gate or
-    // near-return (the full sequence below handles those), and at most a rebase onto Z_0
-    // whose delta keeps binary64's range (f2 > SQUARE_OK on the extended tier), a +-32
-    // rescaling of the extended tier's delta, or a Brent save point of the extended tier.
-    // Each of those is the full sequence's own expressions in its own order, so the state
-    // after either path is the same; the divergent work per lane is a few instructions.
-    const double delta2 = pr * pr + pi * pi;
-    const bool rebase = EXT ? f2 <= delta2 : f2 < delta2;
-    const bool reb = rebase || s.m == p.last;
-    bool common = !(f2 > p.r2) && !(!replaying && s.nucleus >= 0 && s.n == (uint32_t)s.nucleus + 1u);
-    if (B || (EXT && !(f2 > SQUARE_OK))) common = common && !reb;  // bounded radii; sum2 rebase
-    // the judge reads the delta after a rebase on the ordinary tiers (it is then z itself)
-    const double check_r = EXT ? pr : (reb ? fr : s.xr), check_i = EXT ? pi : (reb ? fi : s.xi);
-    bool judge = check_r * check_r + check_i * check_i > RES2 * f2;
-    if (EXT) judge = judge && s.returns < 4;
-    const double dist = fabs(fr - s.sr) + fabs(fi - s.si);
-    if (replaying) {
-    } else if (EXT) {
-      common = common && !(judge && dist < s.near);
-    } else {
-      const bool held = s.hold > 0 && s.n - s.sn < s.hold;  // sn <= n while hold > 0
-      common = common && (judge ? !(dist < s.near) && (s.hold > 0 ? held : !(s.pending || s.n >= s.chk))
-                                : (s.hold > 0 ? held : s.n < s.chk));
-    }
-    if (__builtin_expect(common, 1)) {
-      bool moved = false;
-      if (__builtin_expect(reb, 0)) {  // sample.rs:418-452 without sum2 or TINY (scale is 1)
-        moved = true;
-        s.xr = fr;
-        s.xi = fi;
-        s.m = 0;
-        s.Zr = p.z0r;
-        s.Zi = p.z0i;
-        s.r2a = -1.0;  // no block starts at Z_0 (bla.rs:235-236)
-        s.r2b = -1.0;
-        if (EXT) {
-          s.delta_exp = 0;
-          s.scale = exp2i(s.delta_exp);
-          double factor = exp2i(s.offset_exp - s.delta_exp);
-          s.dc_r = s.ar * factor;
-          s.dc_i = s.ai * factor;
-        }
-      } else if (EXT) {  // sample.rs:453-467
-        const double magnitude = rmax(fabs(s.xr), fabs(s.xi));
-        int32_t k = 0;
-        if (magnitude > HI && s.delta_exp < 0)
-          k = -s.delta_exp < 32 ? -s.delta_exp : 32;
-        else if (magnitude < LO && magnitude != 0.0)
-          k = -32;
-        if (__builtin_expect(k != 0, 0)) {
-          moved = true;
-          double factor = exp2i(-k);
-          s.xr = s.xr * factor;
-          s.xi = s.xi * factor;
-          s.delta_exp = s.delta_exp + k;
-          s.scale = exp2i(s.delta_exp);
-          double f = exp2i(s.offset_exp - s.delta_exp);
-          s.dc_r = s.ar * f;
-          s.dc_i = s.ai * f;
-        }
-      }
-      if (moved) {  // the next iteration's z (sample.rs:331; number.rs:113 on the extended tier)
-        s.fr = EXT ? s.Zr + s.scale * s.xr : s.Zr + s.xr;
-        s.fi = EXT ? s.Zi + s.scale * s.xi : s.Zi + s.xi;
-      } else {
-        s.fr = fr;
-        s.fi = fi;
-      }
-      if (EXT && !replaying && __builtin_expect(s.n >= s.chk, 0)) {  // sample.rs:488-491 / :571-574
-        save_point(s, fr, fi);
-        s.sn = s.n;
-        s.chk = s.chk >= 0x80000000u ? 0xffffffffu : s.chk * 2;
-        relimit(p, s);
-      }
-      return false;
-    }
-  }
   if (__builtin_expect(f2 > p.r2, 0)) {
     res.kind = 0;
     res.n = s.n;
@@ -580,13 +554,18 @@ __device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res
     }
     return true;
   }
-  if (!replaying && __builtin_expect(s.nucleus >= 0, 0) && s.n == (uint32_t)s.nucleus + 1u) {
-    if (s.ct.small()) {
+  if (!replaying && s.gate != NO_GATE && s.n == s.gate) {
+    const int small = s.ct.exact() ? (int)product.get().small() : s.ct.small((int32_t)s.gate - 1);
+    if (small < 0) {
+      res.kind = 3;
+      return true;
+    }
+    if (small) {
       res.kind = 1;
       res.n = s.n;
       return true;
     }
-    s.nucleus = -1;
+    s.gate = NO_GATE;
     relimit(p, s);
   }
   double delta2 = pr * pr + pi * pi;
@@ -613,9 +592,8 @@ __device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res
       s.Zr = p.z0r;
       s.Zi = p.z0i;
       s.r2a = -1.0;  // no block starts at Z_0 (bla.rs:235-236)
-      s.r2b = -1.0;
       if (s.scale < 1.0 / 1e270) {  // TINY, sample.rs:17
-        s.nucleus = -1;
+        s.gate = NO_GATE;
         relimit(p, s);
         if (D) {
           Cx3 v = zero_step_dz(Cx3{s.xr, s.xi, s.delta_exp}, Cx3{s.dr, s.di, s.derivative_exp});
@@ -635,11 +613,7 @@ __device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res
         double2 Z1 = __ldg(p.orbit + 1);
         s.Zr = Z1.x;
         s.Zi = Z1.y;
-        if (L) {
-          double2 rr = __ldg(p.fused + 3);
-          s.r2a = rr.x;
-          s.r2b = rr.y;
-        }
+        if (L) s.r2a = __ldg(p.fused + 3).x;
       }
       double factor = exp2i(s.offset_exp - s.delta_exp);
       s.dc_r = s.ar * factor;
@@ -651,7 +625,6 @@ __device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res
       s.Zr = p.z0r;
       s.Zi = p.z0i;
       s.r2a = -1.0;
-      s.r2b = -1.0;
     }
   } else if (EXT) {
     double magnitude = rmax(fabs(s.xr), fabs(s.xi));
@@ -695,18 +668,18 @@ __device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res
       if (s.n - s.sn >= s.hold) {  // sn <= n while hold > 0
         s.hold = 0;
         s.predicted = false;
-        s.pending = true;
+        await_save(s);
         relimit(p, s);
       }
     } else if (s.n >= s.chk) {
-      s.pending = true;
+      await_save(s);
       relimit(p, s);
     }
     return false;
   }
-  double dist = fabs(fr - s.sr) + fabs(fi - s.si);
+  const double dist = fabs(fr - s.sr) + fabs(fi - s.si), near = near_bound(s);
   if (EXT) {
-    if (s.returns < 4 && dist < s.near) {
+    if (s.returns < 4 && dist < near) {
       if (contracting(p.orbit, p.last, s.m, check_r, check_i, s.ar * exp2i(s.offset_exp),
                       s.ai * exp2i(s.offset_exp), (uint64_t)(s.n - s.sn))) {
         res.kind = 2;
@@ -722,7 +695,7 @@ __device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res
     }
     return false;
   }
-  if (dist < s.near) {
+  if (dist < near) {
     uint32_t period = s.n - s.sn;
     if (s.hold == period && s.mu.below_one()) {
       double mr, mi;
@@ -757,7 +730,7 @@ __device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res
     if (s.n - s.sn < s.hold) return false;
     s.hold = 0;
     s.predicted = false;
-    s.pending = true;
+    await_save(s);
   }
   if (s.pending || s.n >= s.chk) {
     uint64_t np = next_pow2((uint64_t)s.n + 1);
@@ -771,38 +744,174 @@ __device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res
   return false;
 }
 
-// One iteration of the while loop of sample.rs:237-575 for one lane (the allocation-free
-// kernel's form). Returns true when the sample has an outcome (written to res).
-template <bool EXT, bool D, bool L>
-__device__ __forceinline__ bool step(const Params &p, State<EXT> &s, Result &res) {
+// The end of an iteration in which something may have happened: the derivative's rescaling
+// (dbig), an event of the full sequence, a rebase (reb), a rescaling of the delta, a due
+// periodicity check (limit), a near return, a block radius below binary64's squares, or a
+// contraction product leaving its range. Each part tests its own condition exactly.
+template <bool EXT, bool D, bool L, bool B, bool T>
+__device__ __forceinline__ bool settle(const Params &p, State<EXT> &s, Result &res, Entry at, double pr, double pi,
+                                       double fr, double fi, double f2, double delta2, bool reb, bool wild,
+                                       ExactProduct &product, StripeTrace *tr) {
+  if (EXT && D && ((fabs(s.dr) > HI) | (fabs(s.di) > HI))) {  // sample.rs:355-360
+    s.dr = s.dr * LO;
+    s.di = s.di * LO;
+    s.derivative_exp += 32;
+    s.inverse = exp2i(-s.derivative_exp);
+  }
+  const uint32_t end = T ? s.limit : p.max_iter;
+  const bool limit = s.n >= s.lim;
+  bool event = wild | (B && reb);
+  event |= limit && (s.n == s.gate || s.n >= end || (!EXT && s.hold > 0) || (T && s.replaying));
+  event |= (reb && !EXT ? f2 : delta2) > RES2 * f2 && fabs(fr - s.sr) + fabs(fi - s.si) < s.near;
+  if (event) {
+    if (sequence<EXT, D, L, B, T>(p, s, res, make_double2(at.zr, at.zi), pr, pi, fr, fi, f2, product, tr)) return true;
+    if (s.n >= end) {  // the loop's end (sample.rs:237)
+      if (T && s.replaying) {  // sample.rs:576-579: the replay gave up; from what was recorded
+        tr->finish(tr->first_at, tr->first_r, tr->first_i, p.r2, p.stripe_window, p.stripe_freq);
+        res = tr->first;
+      } else {
+        res.kind = 2;
+      }
+      return true;
+    }
+  } else {
+    if (reb) {  // sample.rs:418-452 without sum2 or TINY (scale is 1)
+      s.xr = fr;
+      s.xi = fi;
+      s.m = 0;
+      s.Zr = p.z0r;
+      s.Zi = p.z0i;
+      s.r2a = -1.0;  // no block starts at Z_0 (bla.rs:235-236)
+      if (EXT) {
+        s.delta_exp = 0;
+        s.scale = 1.0;
+        const double factor = exp2i(s.offset_exp);
+        s.dc_r = s.ar * factor;
+        s.dc_i = s.ai * factor;
+      }
+      s.fr = EXT ? s.Zr + s.scale * s.xr : s.Zr + s.xr;  // sample.rs:331; number.rs:113
+      s.fi = EXT ? s.Zi + s.scale * s.xi : s.Zi + s.xi;
+    } else if (EXT) {  // sample.rs:453-467
+      const double magnitude = rmax(fabs(s.xr), fabs(s.xi));
+      int32_t k = 0;
+      if (magnitude > HI && s.delta_exp < 0)
+        k = -s.delta_exp < 32 ? -s.delta_exp : 32;
+      else if (magnitude < LO && magnitude != 0.0)
+        k = -32;
+      if (k != 0) {
+        double factor = exp2i(-k);
+        s.xr = s.xr * factor;
+        s.xi = s.xi * factor;
+        s.delta_exp = s.delta_exp + k;
+        s.scale = exp2i(s.delta_exp);
+        double f = exp2i(s.offset_exp - s.delta_exp);
+        s.dc_r = s.ar * f;
+        s.dc_i = s.ai * f;
+        s.fr = s.Zr + s.scale * s.xr;
+        s.fi = s.Zi + s.scale * s.xi;
+      }
+    }
+    if (limit) {
+      if (EXT) {  // sample.rs:488-491 / :571-574
+        save_point(s, fr, fi);
+        s.sn = s.n;
+        s.chk = s.chk >= 0x80000000u ? 0xffffffffu : s.chk * 2;
+      } else if ((reb ? f2 : delta2) > RES2 * f2) {  // judged, no near return and hold = 0: sample.rs:560-570
+        const uint64_t np = next_pow2((uint64_t)s.n + 1);
+        const uint32_t np32 = np > 0xffffffffull ? 0xffffffffu : (uint32_t)np;
+        s.chk = s.chk > np32 ? s.chk : np32;
+        save_point(s, fr, fi);
+        s.sn = s.n;
+      } else {
+        await_save(s);
+      }
+      relimit(p, s);
+    }
+  }
+  s.on = L && !(T && s.replaying) && block_starts(s);
+  if (!B && !s.on && (event || !s.ct.times(f2, 2))) contraction_wide(s, product, 2.0 * s.fr, 2.0 * s.fi);
+  return false;
+}
+
+// The rest of the iteration after the update (sample.rs:381-575), and the choice of the next
+// operation (s.on: a BLA block). next holds the entry m + 1 prefetched at the iteration's
+// start, right after a plain step; after a block (took) the entry at the new m is loaded
+// here. Returns true when the sample has an outcome. T: the Stripe recorder tr records
+// the iterate, and an escape whose window misses iterates replays them (sample.rs:369-403).
+//
+// A common iteration carries z and chooses the next operation; one test sends every other
+// to settle(). The test may be true without cause, never false with one. Its parts are
+// integer tests on high words where that is enough: binary64 operations issue at half
+// rate, and the iteration holds ~45 of them. Issue slots bound the kernel, and before this
+// form a warp step spent them on a region per condition (a branch and a reconvergence
+// each) and on the contraction's complex product: 21.3 -> 15.1 warp instructions per
+// executed operation and 39.2 -> 28.3 ms a call on the 1920x1080 frame at a 1e-100 nucleus
+// (extended tier, blocks), 4.4 -> 3.1 ms on the 480x270 1e-12 frame without a table. One lane
+// in 8 warp steps is at a rebase, one in 8 at a save point: settle() runs in a third of
+// the warp steps for two or three lanes.
+template <bool EXT, bool D, bool L, bool B = false, bool T = false>
+__device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res, bool took, Entry next,
+                                     ExactProduct &product, StripeTrace *tr = nullptr) {
+  if (L) {
+    if (took) next = load_entry<L>(p, s.m);  // a block moved m by its length
+    s.r2a = next.r2a;
+  }
+  s.Zr = next.zr;
+  s.Zi = next.zi;
+  const double pr = EXT ? s.scale * s.xr : s.xr, pi = EXT ? s.scale * s.xi : s.xi;
+  const double fr = next.zr + pr, fi = next.zi + pi;
+  const double f2 = fr * fr + fi * fi;
+  const double delta2 = pr * pr + pi * pi;
+  if (T) tr->record(s.n, fr, fi);
+  s.fr = fr;  // the next iteration's z, Z[m] + delta with the final m and delta
+  s.fi = fi;
+  const uint32_t f2_hi = (uint32_t)__double2hiint(f2);
+  // |z|^2 outside (1e-290, R^2) on the extended tier (a rebase below takes wide exponents),
+  // not below R^2 on the others, NaN included
+  constexpr uint32_t floor_hi = EXT ? 0x03b8f2b1u : 0u;  // the first high word above 1e-290's
+  const uint32_t top_hi = max((uint32_t)__double2hiint(p.r2), floor_hi);
+  const bool wild = f2_hi - floor_hi >= top_hi - floor_hi;
+  const bool reb = (EXT ? f2 <= delta2 : f2 < delta2) | (s.m == p.last);
+  bool rare = wild | reb | (s.n >= s.lim);
+  // a near return counts where |delta|^2 > 1e-24 |z|^2 (1e-24 > 2^-80), which holds for no
+  // high words further than 80 binades apart (and after a rebase of the ordinary tiers)
+  rare |= (fabs(fr - s.sr) + fabs(fi - s.si) < s.near) & ((uint32_t)__double2hiint(delta2) + (80u << 20) > f2_hi);
+  if (EXT) {
+    // the delta's mantissa outside [2^-32, 2^32), the derivative's above
+    const uint32_t hr = (uint32_t)__double2hiint(s.xr) & 0x7fffffffu, hi = (uint32_t)__double2hiint(s.xi) & 0x7fffffffu;
+    rare |= max(hr, hi) - 0x3df00000u >= 0x04000000u;
+    if (D) rare |= (fabs(s.dr) > HI) | (fabs(s.di) > HI);
+  }
+  if (L) {
+    // block_starts on |delta|^2: its own (x^2) scale^2 rounds alike unless a product falls
+    // below binary64's range, where both lie below any radius^2 of 2^-880 and more
+    s.on = (delta2 < s.r2a) & (s.n + 1u < s.lim);
+    if (EXT) rare |= (uint32_t)__double2hiint(s.r2a) < ((1023u - 880u) << 20);
+    if (T) rare |= s.replaying;
+  }
+  // the contraction's factor of a plain step from here (a block's: apply_block)
+  Magnitude ct = s.ct;
+  if (!B) rare |= !ct.times(f2, 2) & !s.on;
+  if (__builtin_expect(rare, 0))
+    return settle<EXT, D, L, B, T>(p, s, res, next, pr, pi, fr, fi, f2, delta2, reb, wild, product, tr);
+  if (!B && !s.on) s.ct = ct;
+  return false;
+}
+
+// One iteration of the while loop of sample.rs:237-575 for one lane without BLA (the
+// allocation-free kernel's form). Returns true when the sample has an outcome (written to res).
+template <bool EXT, bool D>
+__device__ __forceinline__ bool step(const Params &p, State<EXT> &s, Result &res, ExactProduct &product) {
   if (s.n >= p.max_iter) {
     res.kind = 2;
     return true;
   }
   // next orbit point, loaded before the step's arithmetic so its latency overlaps it
   // (m < last here: a sample that reaches the last point rebases to Z_0)
-  double2 Zn, Rn = make_double2(-1.0, -1.0);
-  if (L) {
-    Zn = __ldg(p.fused + 2 * (s.m + 1));
-    Rn = __ldg(p.fused + 2 * (s.m + 1) + 1);
-  } else {
-    Zn = __ldg(p.orbit + s.m + 1);
-  }
-  uint32_t at = 0;
-  const int lv = L ? find_block(p, s, at) : -1;
-  if (lv >= 0)
-    apply_block<EXT, D>(p, s, lv, at);
-  else
-    plain_update<EXT, D>(s);
-  return post<EXT, D, L>(p, s, res, lv >= 0, Zn, Rn);
+  const Entry next = load_entry<false>(p, s.m + 1);
+  plain_update<EXT, D>(s);
+  return post<EXT, D, false>(p, s, res, false, next, product);
 }
-
-// A lane's BLA block found but not yet applied.
-struct Waiting {
-  bool on;
-  int lv;
-  uint32_t at;
-};
 
 // A warp's reserved queue slots [base, end): one atomic on the queue head takes 32
 // consecutive slots (one tile), which the warp then hands to its idle lanes in order, so
@@ -836,62 +945,40 @@ struct Reservation {
   }
 };
 
-// One iteration for the active lanes of a warp (every lane of the warp calls it). A lane
-// whose next operation is a BLA block waits until at least defer/32 of the warp's busy
-// lanes wait or no lane steps plainly; the waiting lanes then apply their blocks together. The warp
-// runs the block path for many lanes at a time instead of for one or two lanes on
+// One iteration for the lanes of a warp that hold a sample (`held`, warp-uniform; every lane
+// of the warp calls it). A lane whose next operation is a BLA block waits until thr lanes
+// wait or no lane steps plainly; the waiting lanes then apply their blocks together. The
+// warp runs the block path for many lanes at a time instead of for one or two lanes on
 // nearly every iteration, and each lane's own sequence of operations is unchanged.
 template <bool EXT, bool D, bool L, bool B = false, bool T = false>
-__device__ __forceinline__ bool warp_step(const Params &p, State<EXT> &s, Result &res, bool active, Waiting &w,
-                                          uint32_t defer, StripeTrace *tr = nullptr) {
-  bool upd = false, took = false, done = false;
-  double2 Zn = make_double2(0.0, 0.0), Rn = make_double2(-1.0, -1.0);
-  if (active && !w.on) {
-    if (s.n >= (T ? s.limit : p.max_iter)) {
-      if (T && s.replaying) {  // sample.rs:576-579: the replay gave up; from what was recorded
-        tr->finish(tr->first_at, tr->first_r, tr->first_i, p.r2, p.stripe_window, p.stripe_freq);
-        res = tr->first;
-      } else {
-        res.kind = 2;
-      }
-      done = true;
-    } else {
-      if (L) {
-        Zn = __ldg(p.fused + 2 * (s.m + 1));
-        Rn = __ldg(p.fused + 2 * (s.m + 1) + 1);
-      } else {
-        Zn = __ldg(p.orbit + s.m + 1);
-      }
-      // a lane that finds a block waits; its level is searched when the waiting lanes
-      // apply their blocks together (nothing the search reads changes while it waits)
-      if (L && !(T && s.replaying) && block_starts(s)) {
-        w.on = true;
-      } else {
-        plain_update<EXT, D, B>(s, p.q);
-        upd = true;
-      }
-    }
+__device__ __forceinline__ bool warp_step(const Params &p, State<EXT> &s, Result &res, bool active, unsigned held,
+                                          uint32_t thr, ExactProduct &product, StripeTrace *tr = nullptr) {
+  bool upd = active, took = false;
+  Entry next{0.0, 0.0, -1.0};
+  if (L) upd = active && !s.on;
+  if (upd) {
+    next = load_entry<L>(p, s.m + 1);
+    plain_update<EXT, D, B>(s, p.q);
   }
   if (L) {
-    const unsigned FULL = 0xffffffffu;
-    const unsigned waiting = __ballot_sync(FULL, w.on);
-    const unsigned stepping = __ballot_sync(FULL, upd);
-    // the threshold is `defer` of 32 lanes, scaled to the lanes still busy (waiting or
-    // stepping): once the queue runs dry and lanes go idle, a fixed threshold would hold
-    // every waiting lane until the last plain-stepping lane finds a block
-    const uint32_t busy = (uint32_t)__popc(waiting | stepping);
-    const uint32_t thr = max(1u, (busy * defer) >> 5);
-    if (waiting && ((uint32_t)__popc(waiting) >= thr || !stepping) && w.on) {
-      w.lv = block_level(p, s, w.at);
+    const unsigned waiting = __ballot_sync(0xffffffffu, active && s.on);
+    if (((uint32_t)__popc(waiting) >= thr || waiting == held) && active && s.on) {
+      uint32_t at;
+      const int lv = block_level(p, s, at);
       if (T)  // sample.rs:267-281: the block start, for a later replay
-        tr->snap(StripeSnap{s.m, s.n, s.xr, s.xi, s.delta_exp, s.scale, s.dc_r, s.dc_i, 0}, s.n + (2u << w.lv));
-      apply_block<EXT, D>(p, s, w.lv, w.at);
-      w.on = false;
+        tr->snap(StripeSnap{s.m, s.n, s.xr, s.xi, s.delta_exp, s.scale, s.dc_r, s.dc_i, 0}, s.n + (2u << lv));
+      apply_block<EXT, D>(p, s, lv, at, product);
       upd = took = true;
     }
   }
-  if (upd) done = post<EXT, D, L, B, T>(p, s, res, took, Zn, Rn, tr);
-  return done;
+  return upd && post<EXT, D, L, B, T>(p, s, res, took, next, product, tr);
+}
+
+// The threshold of warp_step: defer of 32 lanes, scaled to the lanes that hold a sample
+// (once the queue runs dry lanes go idle, and a fixed threshold would hold every
+// waiting lane until the last plain-stepping lane finds a block).
+__device__ __forceinline__ uint32_t threshold(unsigned held, uint32_t defer) {
+  return max(1u, ((uint32_t)__popc(held) * defer) >> 5);
 }
 
 // Series::eval (series.rs:247-271): Horner on x = dc / rho for p = sum b_k x^(k-1) and
@@ -995,7 +1082,6 @@ __device__ __forceinline__ void start_sample(const Params &p, State<EXT> &s, boo
   s.Zr = p.z0r;
   s.Zi = p.z0i;
   s.r2a = -1.0;
-  s.r2b = -1.0;
   s.fr = EXT ? p.z0r + s.scale * 0.0 : p.z0r + 0.0;  // z of the first iteration
   s.fi = EXT ? p.z0i + s.scale * 0.0 : p.z0i + 0.0;
   save_point(s, 0.0, 0.0);
@@ -1012,8 +1098,9 @@ __device__ __forceinline__ void start_sample(const Params &p, State<EXT> &s, boo
   s.qi = 0.0;
   s.qstep = 0.0;
   s.adc = L ? sqrt(s.ar * s.ar + s.ai * s.ai) : 0.0;
-  s.nucleus = (int32_t)p.nucleus;
-  s.ct.reset();
+  s.gate = p.nucleus >= 0 ? (uint32_t)p.nucleus + 1u : NO_GATE;
+  s.ct.reset((int32_t)p.nucleus);
+  s.on = false;
   if (!keep_counts) {
     s.blocks = 0;
     s.skipped = 0;
@@ -1026,32 +1113,26 @@ __device__ __forceinline__ void start_sample(const Params &p, State<EXT> &s, boo
     const uint32_t m = p.series_n;
     s.m = m;
     s.n = m;
-    if (L) {
-      const double2 Z = __ldg(p.fused + 2 * m), R = __ldg(p.fused + 2 * m + 1);
-      s.Zr = Z.x;
-      s.Zi = Z.y;
-      s.r2a = R.x;
-      s.r2b = R.y;
-    } else {
-      const double2 Z = __ldg(p.orbit + m);
-      s.Zr = Z.x;
-      s.Zi = Z.y;
-    }
+    const Entry at = load_entry<L>(p, m);
+    s.Zr = at.zr;
+    s.Zi = at.zi;
+    s.r2a = at.r2a;
     s.fr = s.Zr + s.xr;
     s.fi = s.Zi + s.xi;
     save_point(s, s.Zr + s.xr, s.Zi + s.xi);
     s.sn = m;
     const uint64_t np = next_pow2((uint64_t)m + 1);
     s.chk = np > 16 ? (uint32_t)np : 16u;
-    s.nucleus = -1;
+    s.gate = NO_GATE;
   }
   if (B) {  // sample.rs:221-229: radii from zero; a bounded render has no nucleus heuristic
     s.e = 0.0;
     s.ed = 0.0;
     s.rc = 16.0 * U * (fabs(s.ar) + fabs(s.ai)) + 1e-300;
-    s.nucleus = -1;
+    s.gate = NO_GATE;
   }
   relimit(p, s);
+  if (L && !EXT && use_series && p.series_n > 0) s.on = block_starts(s);
 }
 
 // Column encoder (store.rs:66-112, Bound absent) and raw state.
@@ -1188,15 +1269,15 @@ struct TraceSlot<true> {
 // ms; without BLA the 480x270 1e-12 frame ran 3% slower, so those variants encode as they
 // finish).
 template <bool EXT, bool D, bool L, bool S = false, bool B = false, bool T = false>
-__global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(Params p) {
+__global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(const __grid_constant__ Params p) {
   const unsigned FULL = 0xffffffffu;
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt = (1u << lane) - 1u;
   State<EXT> s;
   Result res;
-  Waiting w{false, -1, 0};
   bool active = false, exhausted = false;
   Reservation slots;
+  ExactProduct product;
   TraceSlot<T> trace;
   StripeTrace *tr = trace.get();
   uint64_t t0 = p.deadline_ns ? globaltimer() : 0;
@@ -1206,6 +1287,7 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(Pa
   // on a first run from the series (> 0); after an unresolved first run retried from zero,
   // prefix - max_iter, so that the first run counts max_iter - prefix.
   int64_t bias = 0;
+  uint32_t blocks0 = 0, skipped0 = 0;  // S: the counts the run from zero started with
   auto finish = [&](uint32_t idx, const Result &r, uint64_t nblocks, uint64_t nskipped, double sh) {
     put<B, T, L && !B && !T>(p, idx, r, T && r.kind == 0 ? tr->value : 0.0f);
     uint64_t spent = (uint64_t)((int64_t)(r.kind == 2 ? p.max_iter : r.n) - bias);
@@ -1221,6 +1303,18 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(Pa
     }
     iters += spent;
     n_samples += 1;
+  };
+  // an unresolved series start retries from zero, keeping the nucleus heuristic
+  // (grid.rs:637-642); its count and blocks carry over
+  auto retry = [&]() {
+    bias -= (int64_t)p.max_iter;
+    blocks0 = s.blocks;
+    skipped0 = s.skipped;
+    start_sample<EXT, D, L, B>(p, s, false, true);
+    if (T) {  // grid.rs:638
+      tr->begin();
+      tr->start(s.n);
+    }
   };
   for (;;) {
     unsigned need = __ballot_sync(FULL, !active);
@@ -1247,11 +1341,19 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(Pa
         if (rank < take) {
           int got = init<EXT, D, L, S, B>(p, slot, s, res);
           if (got == 1) {
-            active = true;
-            if (S) bias = p.series_n;
+            if (S) {
+              bias = p.series_n;
+              blocks0 = skipped0 = 0;
+            }
             if (T) {  // Job::one (grid.rs:630) and the loop's start (sample.rs:235)
               tr->begin();
               tr->start(s.n);
+            }
+            if (S && bias > 0 && s.n >= p.max_iter) retry();
+            active = s.n < p.max_iter;
+            if (!active) {  // no iteration to run
+              res.kind = 2;
+              finish(s.idx, res, s.blocks, s.skipped, s.shift);
             }
           } else if (got == 2) {
             finish(s.idx, res, 0, 0, 0.0);
@@ -1260,21 +1362,37 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(Pa
       }
       need = __ballot_sync(FULL, !active);
     }
-    if (!__any_sync(FULL, active)) break;
-    if (warp_step<EXT, D, L, B, T>(p, s, res, active, w, p.defer, tr)) {
-      if (S && bias > 0 && res.kind == 2) {
-        // an unresolved series start retries from zero, keeping the nucleus heuristic
-        // (grid.rs:637-642); its count and blocks carry over
-        bias -= (int64_t)p.max_iter;
-        start_sample<EXT, D, L, B>(p, s, false, true);
-        if (T) {  // grid.rs:638
-          tr->begin();
-          tr->start(s.n);
+    // the lanes step until one of them finishes
+    const unsigned held = __ballot_sync(FULL, active);
+    if (!held) break;
+    const uint32_t thr = threshold(held, p.defer);
+    unsigned ended = 0;
+    do {
+      bool done = warp_step<EXT, D, L, B, T>(p, s, res, active, held, thr, product, tr);
+      if (__builtin_expect(done, 0)) {
+        if (S && bias > 0 && res.kind == 2) {
+          retry();
+          done = false;
+        } else if (res.kind == 3) {  // once more, for Contraction's own product
+          start_sample<EXT, D, L, B>(p, s, false, S);
+          if (S) {
+            s.blocks = blocks0;
+            s.skipped = skipped0;
+          }
+          if (T) {
+            tr->begin();
+            tr->start(s.n);
+          }
+          s.ct.take_exact();
+          product.reset();
+          done = false;
         }
-      } else {
-        finish(s.idx, res, s.blocks, s.skipped, s.shift);
-        active = false;
       }
+      ended = __ballot_sync(FULL, done);
+    } while (!ended);
+    if ((ended >> lane) & 1u) {
+      finish(s.idx, res, s.blocks, s.skipped, s.shift);
+      active = false;
     }
   }
   // warp reduction of the counters, one atomic per warp
@@ -1344,10 +1462,10 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks)
   const unsigned lt = (1u << lane) - 1u;
   State<EXT> s;
   Result res;
-  Waiting w{false, -1, 0};
   bool active = false, exhausted = false;
   uint32_t job = 0, counted = 0xffffffffu;
   Reservation slots;
+  ExactProduct product;
   LaneCounters lc;
   lc.clear();
   // the BLA variants store a finished sample's raw state; encode_jobs_kernel computes the
@@ -1386,15 +1504,31 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks)
           job = job_of(starts, njobs, slot);
           const Params &p = jobs[job];
           int got = init<EXT, D, L>(p, slot - __ldg(starts + job), s, res);
-          if (got == 1) active = true;
-          else if (got == 2) finish(p, s.idx, res, 0, 0);
+          active = got == 1 && s.n < p.max_iter;
+          if (got != 0 && !active) {  // settled, or no iteration to run
+            if (got == 1) res.kind = 2;
+            finish(p, s.idx, res, 0, 0);
+          }
         }
       }
       need = __ballot_sync(FULL, !active);
     }
-    if (!__any_sync(FULL, active)) break;
+    const unsigned held = __ballot_sync(FULL, active);
+    if (!held) break;
+    const uint32_t thr = threshold(held, defer);
     const Params &p = jobs[job];
-    if (warp_step<EXT, D, L>(p, s, res, active, w, defer)) {
+    unsigned ended = 0;
+    do {
+      bool done = warp_step<EXT, D, L>(p, s, res, active, held, thr, product);
+      if (__builtin_expect(done && res.kind == 3, 0)) {  // once more, for Contraction's own product
+        start_sample<EXT, D, L, false>(p, s, false, false);
+        s.ct.take_exact();
+        product.reset();
+        done = false;
+      }
+      ended = __ballot_sync(FULL, done);
+    } while (!ended);
+    if ((ended >> lane) & 1u) {
       finish(p, s.idx, res, s.blocks, s.skipped);
       active = false;
     }
