@@ -106,10 +106,14 @@ struct fdc_ctx {
 
 // Persistent grid of a plain-form kernel: the occupancy limit, or fewer blocks per SM
 // when the tuning asks for fewer.
-// Lanes a warp gathers before applying BLA blocks (fdc_tuning.defer; 0: per variant).
-static uint32_t defer_for(const fdc_ctx *ctx, bool ext) {
+// Lanes a warp gathers before applying BLA blocks (fdc_tuning.defer; 0: per variant). The
+// extended tier's blocks carry renormalisations and gather more lanes. Kernel ms over 4, 6,
+// 8, 10, 12, 16: 1920x1080 at a 1e-100 nucleus, extended tier 27.2 25.6 24.3 23.6 23.3 24.1;
+// 1280x720 on the Fixed tier 11.7 12.1 12.5 12.6 13.1 14.2.
+// The precision form's own defaults are 12 and 8.
+static uint32_t defer_for(const fdc_ctx *ctx, bool ext, bool f32) {
   if (ctx->tune.defer > 0) return ctx->tune.defer;
-  return ext ? 12u : 8u;
+  return ext ? 12u : (f32 ? 8u : 4u);
 }
 
 // The tiles of a window, nearest to its centre first (squared distance of the tile's
@@ -635,7 +639,7 @@ fdc_status prepare(fdc_ctx *ctx, const OrbitDev &o, const fdc_job &j, fdk::Param
     if (!p.tile_order) return fail(ctx, FDC_DEVICE_ERROR, "device memory for the tile order");
   }
   p.deadline_ns = j.deadline_ms > 0 ? (uint64_t)(j.deadline_ms * 1e6) : 0;
-  p.defer = defer_for(ctx, p.tier == FDC_TIER_SCALED);
+  p.defer = defer_for(ctx, p.tier == FDC_TIER_SCALED, (j.flags & FDC_F32) != 0);
 
   p.orbit32 = o.z32;
   return FDC_OK;
@@ -1353,12 +1357,12 @@ fdc_status fdc_batch_create(fdc_ctx *ctx, const fdc_job *jobs, const fdc_out *ou
     uint32_t n = (uint32_t)g.order.size();
     if (g.f32) {
       e = fdk::launch_f32_batch(g.jobs, g.starts, n, g.total, q, c, g.deriv, g.bla, ctx->sm_count,
-                                (int)ctx->tune.blocks_per_sm, defer_for(ctx, g.ext), ctx->stream,
+                                (int)ctx->tune.blocks_per_sm, defer_for(ctx, g.ext, true), ctx->stream,
                                 ctx->blocks_per_sm_batch_f32);
     } else {
       int variant = 0;
       void *fn = pick_batch_kernel(g.ext, g.deriv, g.bla, variant);
-      uint32_t defer = defer_for(ctx, g.ext);
+      uint32_t defer = defer_for(ctx, g.ext, false);
       void *args[] = {&g.jobs, &g.starts, &n, &g.total, &q, &c, &defer};
       e = cudaLaunchKernel(fn, dim3(grid_blocks(ctx, ctx->blocks_per_sm_batch[variant])), dim3(128), args, 0,
                            ctx->stream);
