@@ -381,9 +381,7 @@ struct ExactProduct {
 // where the sample is iterated again for it.
 template <bool EXT>
 __device__ __forceinline__ void contraction_wide(State<EXT> &s, ExactProduct &product, double r, double i) {
-  if (s.gate == NO_GATE)
-    s.ct.reset(0);  // no longer asked for
-  else if (s.ct.exact())
+  if (s.ct.exact())
     product.multiply(r, i);
   else
     s.ct.times_wide(r, i);
@@ -436,9 +434,10 @@ __device__ __forceinline__ Entry load_entry(const Params &p, uint32_t m) {
 // of delta and derivative) folded into one of each result. Scaling by a power of two is
 // exact and a normalised value does not depend on how it was scaled before, so the steps
 // around the block can be left out wherever no product counts that leaves binary64's
-// normal range, in this scaling or in the normalised one (within 2^100 of it): the inputs
-// in 2^+-100, every part of the results in [2^-300, 2^900) (a product below 2^-900 then
-// vanishes in the sum either way), and where B's terms are scaled below 2^-900, B below 2^300.
+// normal range, in this scaling or in the normalised one: the inputs in [2^-400, 2^100) (a
+// rebase near a nucleus leaves a small mantissa for a few iterations), every part of the
+// results in [2^-300, 2^500) (a product below binary64's normal range then vanishes in the
+// sum either way), and where B's terms are scaled below 2^-900, B below 2^300.
 // False, with nothing changed, for any other block (a zero part among them) and for a
 // mantissa so close to 2 that floor(log2) rounds up; apply_block then runs the full steps.
 // Before, the normalisations were half of a block's instructions: with the level search's
@@ -459,17 +458,17 @@ __device__ __forceinline__ bool block_quick(State<true> &s, double2 A, double2 B
     hi = max(hi, dh);
     far |= s.derivative_exp > 900;
   }
-  bool ok = lo >= ONE - (100u << 20) && hi < ONE + (100u << 20) &&
+  bool ok = lo >= ONE - (400u << 20) && hi < ONE + (100u << 20) &&
             (!far || max(magnitude_hi(B.x), magnitude_hi(B.y)) < ONE + (300u << 20));
   const double xr = A.x * s.xr - A.y * s.xi + B.x * s.dc_r - B.y * s.dc_i;
   const double xi = A.x * s.xi + A.y * s.xr + B.x * s.dc_i + B.y * s.dc_r;
   const uint32_t xrh = magnitude_hi(xr), xih = magnitude_hi(xi), rx = max(xrh, xih);
-  ok &= min(xrh, xih) >= ONE - (300u << 20) && rx < ONE + (900u << 20) && (rx & 0xfffffu) != 0xfffffu;
+  ok &= min(xrh, xih) >= ONE - (300u << 20) && rx < ONE + (500u << 20) && (rx & 0xfffffu) != 0xfffffu;
   if (D) {
     const double dr = A.x * s.dr - A.y * s.di + B.x * s.inverse;
     const double di = A.x * s.di + A.y * s.dr + B.y * s.inverse;
     const uint32_t drh = magnitude_hi(dr), dih = magnitude_hi(di), rd = max(drh, dih);
-    ok &= min(drh, dih) >= ONE - (300u << 20) && rd < ONE + (900u << 20) && (rd & 0xfffffu) != 0xfffffu;
+    ok &= min(drh, dih) >= ONE - (300u << 20) && rd < ONE + (500u << 20) && (rd & 0xfffffu) != 0xfffffu;
     if (!ok) return false;
     const int k = (int)(rd >> 20) - 1023;
     const double f = pow2(-k);
@@ -505,7 +504,8 @@ __device__ __forceinline__ void apply_block(const Params &p, State<EXT> &s, int 
   const Block4 c = load_block(p.bla_coef + 2 * b);
   const double2 A = c.a, B = c.b;
   const uint32_t len = 2u << lv;
-  if (__builtin_expect(!s.ct.times(A.x * A.x + A.y * A.y, 0), 0)) contraction_wide(s, product, A.x, A.y);
+  if (__builtin_expect(!s.ct.times(A.x * A.x + A.y * A.y, 0) && s.gate != NO_GATE, 0))
+    contraction_wide(s, product, A.x, A.y);
   if (!EXT && s.hold > 0) s.mu.multiply(A.x, A.y);
   if (!BlockQuick<EXT, D>::run(s, A, B)) {
     if (EXT) {
@@ -915,7 +915,7 @@ __device__ __forceinline__ bool settle(const Params &p, State<EXT> &s, Result &r
     }
   }
   s.on = L && !(T && s.replaying) && block_starts(s);
-  if (!B && !s.on && (event || !s.ct.times(f2, 2))) contraction_wide(s, product, 2.0 * s.fr, 2.0 * s.fi);
+  if (!B && !s.on && s.gate != NO_GATE && (event || !s.ct.times(f2, 2))) contraction_wide(s, product, 2.0 * s.fr, 2.0 * s.fi);
   return false;
 }
 
@@ -977,7 +977,7 @@ __device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res
   }
   // the contraction's factor of a plain step from here (a block's: apply_block)
   Magnitude ct = s.ct;
-  if (!B) rare |= !ct.times(f2, 2) & !s.on;
+  if (!B) rare |= !ct.times(f2, 2) & !s.on & (s.gate != NO_GATE);
   if (__builtin_expect(rare, 0))
     return settle<EXT, D, L, B, T>(p, s, res, next, pr, pi, fr, fi, f2, delta2, reb, wild, product, tr);
   if (!B && !s.on) s.ct = ct;
