@@ -434,10 +434,11 @@ __device__ __forceinline__ Entry load_entry(const Params &p, uint32_t m) {
 // of delta and derivative) folded into one of each result. Scaling by a power of two is
 // exact and a normalised value does not depend on how it was scaled before, so the steps
 // around the block can be left out wherever no product counts that leaves binary64's
-// normal range, in this scaling or in the normalised one: the inputs in [2^-400, 2^100) (a
-// rebase near a nucleus leaves a small mantissa for a few iterations), every part of the
-// results in [2^-300, 2^500) (a product below binary64's normal range then vanishes in the
-// sum either way), and where B's terms are scaled below 2^-900, B below 2^300.
+// normal range, in this scaling or in the normalised one: the inputs in [2^-500, 2^100) (a
+// rebase near a nucleus leaves a mantissa down to 1e-145 for a few iterations), every part
+// of the results in [2^-600, 2^500) (a product below binary64's normal range in either
+// scaling then vanishes in the sum, and an overflow in either shows in one part at least),
+// and where dc or 1 is scaled below 2^-900, B's terms 80 binades below the results.
 // False, with nothing changed, for any other block (a zero part among them) and for a
 // mantissa so close to 2 that floor(log2) rounds up; apply_block then runs the full steps.
 // Before, the normalisations were half of a block's instructions: with the level search's
@@ -451,24 +452,27 @@ __device__ __forceinline__ bool block_quick(State<true> &s, double2 A, double2 B
   constexpr uint32_t ONE = 1023u << 20;
   const uint32_t xh = max(magnitude_hi(s.xr), magnitude_hi(s.xi));
   uint32_t lo = xh, hi = xh;
-  bool far = s.offset_exp - s.delta_exp < -900;
   if (D) {
     const uint32_t dh = max(magnitude_hi(s.dr), magnitude_hi(s.di));
     lo = min(lo, dh);
     hi = max(hi, dh);
-    far |= s.derivative_exp > 900;
   }
-  bool ok = lo >= ONE - (400u << 20) && hi < ONE + (100u << 20) &&
-            (!far || max(magnitude_hi(B.x), magnitude_hi(B.y)) < ONE + (300u << 20));
+  bool ok = lo >= ONE - (500u << 20) && hi < ONE + (100u << 20);
   const double xr = A.x * s.xr - A.y * s.xi + B.x * s.dc_r - B.y * s.dc_i;
   const double xi = A.x * s.xi + A.y * s.xr + B.x * s.dc_i + B.y * s.dc_r;
   const uint32_t xrh = magnitude_hi(xr), xih = magnitude_hi(xi), rx = max(xrh, xih);
-  ok &= min(xrh, xih) >= ONE - (300u << 20) && rx < ONE + (500u << 20) && (rx & 0xfffffu) != 0xfffffu;
+  const uint32_t low = min(xrh, xih);
+  ok &= low >= ONE - (600u << 20) && rx < ONE + (500u << 20) && (rx & 0xfffffu) != 0xfffffu;
+  const int off = s.offset_exp - s.delta_exp;  // dc's parts are below 2^20 2^off
+  if (off < -900) ok &= (int)(max(magnitude_hi(B.x), magnitude_hi(B.y)) >> 20) + off + 100 <= (int)(low >> 20);
   if (D) {
     const double dr = A.x * s.dr - A.y * s.di + B.x * s.inverse;
     const double di = A.x * s.di + A.y * s.dr + B.y * s.inverse;
     const uint32_t drh = magnitude_hi(dr), dih = magnitude_hi(di), rd = max(drh, dih);
-    ok &= min(drh, dih) >= ONE - (300u << 20) && rd < ONE + (500u << 20) && (rd & 0xfffffu) != 0xfffffu;
+    const uint32_t dlow = min(drh, dih);
+    ok &= dlow >= ONE - (600u << 20) && rd < ONE + (500u << 20) && (rd & 0xfffffu) != 0xfffffu;
+    if (s.derivative_exp > 900)
+      ok &= (int64_t)(max(magnitude_hi(B.x), magnitude_hi(B.y)) >> 20) - s.derivative_exp + 80 <= (int64_t)(dlow >> 20);
     if (!ok) return false;
     const int k = (int)(rd >> 20) - 1023;
     const double f = pow2(-k);
