@@ -554,10 +554,21 @@ __device__ __forceinline__ void apply_block(const Params &p, State<EXT> &s, int 
   s.skipped += len;
 }
 
+template <bool EXT, bool L>
+__device__ __forceinline__ void enter(const Params &p, State<EXT> &s) {
+  const Entry at = load_entry<L>(p, s.m);
+  s.Zr = at.zr;
+  s.Zi = at.zi;
+  if (L) s.r2a = at.r2a;
+}
+
 // One ordinary step (sample.rs:331-380; number.rs:92-124): z = Z[m] + delta is carried
 // from the end of the previous iteration in (fr, fi).
-template <bool EXT, bool D, bool B = false>
-__device__ __forceinline__ void plain_update(State<EXT> &s, const double *__restrict__ q = nullptr) {
+// The entry at the new m is loaded into the state between the delta's update, which uses the
+// old one, and the derivative's, which covers the load's latency.
+template <bool EXT, bool D, bool L, bool B = false>
+__device__ __forceinline__ void plain_update(const Params &p, State<EXT> &s) {
+  const double *__restrict__ q = p.q;
   const double fr = s.fr, fi = s.fi;
   if (!EXT && s.hold > 0) s.mu.multiply(2.0 * fr, 2.0 * fi);
   if (B) {  // sample.rs:338-350: the radii through this step, from the state before it
@@ -572,11 +583,6 @@ __device__ __forceinline__ void plain_update(State<EXT> &s, const double *__rest
     const double w = af + qm + 2.0 * U * af;  // >= |A_m + delta|
     s.e = (s.e * (2.0 * w + s.e) + rho) * SAFE;
   }
-  if (D) {
-    double t = 2.0 * (fr * s.dr - fi * s.di) + s.inverse;
-    s.di = 2.0 * (fr * s.di + fi * s.dr);
-    s.dr = t;
-  }
   const double wr = s.xr, wi = s.xi, zr = s.Zr, zi = s.Zi;
   if (EXT) {  // number.rs:109-124
     s.xr = 2.0 * (zr * wr - zi * wi) + s.scale * (wr * wr - wi * wi) + s.dc_r;
@@ -587,6 +593,12 @@ __device__ __forceinline__ void plain_update(State<EXT> &s, const double *__rest
   }
   s.m += 1;
   s.n += 1;
+  enter<EXT, L>(p, s);
+  if (D) {
+    double t = 2.0 * (fr * s.dr - fi * s.di) + s.inverse;
+    s.di = 2.0 * (fr * s.di + fi * s.dr);
+    s.dr = t;
+  }
 }
 
 // The full sequence after an update (sample.rs:381-575) for iterations in which some event
@@ -839,7 +851,7 @@ __device__ __forceinline__ bool sequence(const Params &p, State<EXT> &s, Result 
 // periodicity check (limit), a near return, a block radius below binary64's squares, or a
 // contraction product leaving its range. Each part tests its own condition exactly.
 template <bool EXT, bool D, bool L, bool B, bool T>
-__device__ __forceinline__ bool settle(const Params &p, State<EXT> &s, Result &res, Entry at, double pr, double pi,
+__device__ __forceinline__ bool settle(const Params &p, State<EXT> &s, Result &res, double pr, double pi,
                                        double fr, double fi, double f2, double delta2, bool reb, bool wild,
                                        ExactProduct &product, StripeTrace *tr) {
   if (EXT && D && ((fabs(s.dr) > HI) | (fabs(s.di) > HI))) {  // sample.rs:355-360
@@ -854,7 +866,7 @@ __device__ __forceinline__ bool settle(const Params &p, State<EXT> &s, Result &r
   event |= limit && (s.n == s.gate || s.n >= end || (!EXT && s.hold > 0) || (T && s.replaying));
   event |= (reb && !EXT ? f2 : delta2) > RES2 * f2 && fabs(fr - s.sr) + fabs(fi - s.si) < s.near;
   if (event) {
-    if (sequence<EXT, D, L, B, T>(p, s, res, make_double2(at.zr, at.zi), pr, pi, fr, fi, f2, product, tr)) return true;
+    if (sequence<EXT, D, L, B, T>(p, s, res, make_double2(s.Zr, s.Zi), pr, pi, fr, fi, f2, product, tr)) return true;
     if (s.n >= end) {  // the loop's end (sample.rs:237)
       if (T && s.replaying) {  // sample.rs:576-579: the replay gave up; from what was recorded
         tr->finish(tr->first_at, tr->first_r, tr->first_i, p.r2, p.stripe_window, p.stripe_freq);
@@ -924,9 +936,7 @@ __device__ __forceinline__ bool settle(const Params &p, State<EXT> &s, Result &r
 }
 
 // The rest of the iteration after the update (sample.rs:381-575), and the choice of the next
-// operation (s.on: a BLA block). next holds the entry m + 1 prefetched at the iteration's
-// start, right after a plain step; after a block (took) the entry at the new m is loaded
-// here. Returns true when the sample has an outcome. T: the Stripe recorder tr records
+// operation (s.on: a BLA block), with the entry at the new m in the state. Returns true when the sample has an outcome. T: the Stripe recorder tr records
 // the iterate, and an escape whose window misses iterates replays them (sample.rs:369-403).
 //
 // A common iteration carries z and chooses the next operation; one test sends every other
@@ -940,16 +950,10 @@ __device__ __forceinline__ bool settle(const Params &p, State<EXT> &s, Result &r
 // in 8 warp steps is at a rebase, one in 8 at a save point: settle() runs in a third of
 // the warp steps for two or three lanes.
 template <bool EXT, bool D, bool L, bool B = false, bool T = false>
-__device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res, bool took, Entry next,
-                                     ExactProduct &product, StripeTrace *tr = nullptr) {
-  if (L) {
-    if (took) next = load_entry<L>(p, s.m);  // a block moved m by its length
-    s.r2a = next.r2a;
-  }
-  s.Zr = next.zr;
-  s.Zi = next.zi;
+__device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res, ExactProduct &product,
+                                     StripeTrace *tr = nullptr) {
   const double pr = EXT ? s.scale * s.xr : s.xr, pi = EXT ? s.scale * s.xi : s.xi;
-  const double fr = next.zr + pr, fi = next.zi + pi;
+  const double fr = s.Zr + pr, fi = s.Zi + pi;
   const double f2 = fr * fr + fi * fi;
   const double delta2 = pr * pr + pi * pi;
   if (T) tr->record(s.n, fr, fi);
@@ -983,7 +987,7 @@ __device__ __forceinline__ bool post(const Params &p, State<EXT> &s, Result &res
   Magnitude ct = s.ct;
   if (!B) rare |= !ct.times(f2, 2) & !s.on & (s.gate != NO_GATE);
   if (__builtin_expect(rare, 0))
-    return settle<EXT, D, L, B, T>(p, s, res, next, pr, pi, fr, fi, f2, delta2, reb, wild, product, tr);
+    return settle<EXT, D, L, B, T>(p, s, res, pr, pi, fr, fi, f2, delta2, reb, wild, product, tr);
   if (!B && !s.on) s.ct = ct;
   return false;
 }
@@ -996,11 +1000,8 @@ __device__ __forceinline__ bool step(const Params &p, State<EXT> &s, Result &res
     res.kind = 2;
     return true;
   }
-  // next orbit point, loaded before the step's arithmetic so its latency overlaps it
-  // (m < last here: a sample that reaches the last point rebases to Z_0)
-  const Entry next = load_entry<false>(p, s.m + 1);
-  plain_update<EXT, D>(s);
-  return post<EXT, D, false>(p, s, res, false, next, product);
+  plain_update<EXT, D, false>(p, s);  // m < last here: a sample that reaches the last point rebases to Z_0
+  return post<EXT, D, false>(p, s, res, product);
 }
 
 // A warp's reserved queue slots [base, end): one atomic on the queue head takes 32
@@ -1043,13 +1044,9 @@ struct Reservation {
 template <bool EXT, bool D, bool L, bool B = false, bool T = false>
 __device__ __forceinline__ bool warp_step(const Params &p, State<EXT> &s, Result &res, bool active, unsigned held,
                                           uint32_t thr, ExactProduct &product, StripeTrace *tr = nullptr) {
-  bool upd = active, took = false;
-  Entry next{0.0, 0.0, -1.0};
+  bool upd = active;
   if (L) upd = active && !s.on;
-  if (upd) {
-    next = load_entry<L>(p, s.m + 1);
-    plain_update<EXT, D, B>(s, p.q);
-  }
+  if (upd) plain_update<EXT, D, L, B>(p, s);
   if (L) {
     const unsigned waiting = __ballot_sync(0xffffffffu, active && s.on);
     if (((uint32_t)__popc(waiting) >= thr || waiting == held) && active && s.on) {
@@ -1058,10 +1055,11 @@ __device__ __forceinline__ bool warp_step(const Params &p, State<EXT> &s, Result
       if (T)  // sample.rs:267-281: the block start, for a later replay
         tr->snap(StripeSnap{s.m, s.n, s.xr, s.xi, s.delta_exp, s.scale, s.dc_r, s.dc_i, 0}, s.n + (2u << lv));
       apply_block<EXT, D>(p, s, lv, at, product);
-      upd = took = true;
+      enter<EXT, L>(p, s);
+      upd = true;
     }
   }
-  return upd && post<EXT, D, L, B, T>(p, s, res, took, next, product, tr);
+  return upd && post<EXT, D, L, B, T>(p, s, res, product, tr);
 }
 
 // The threshold of warp_step: defer of 32 lanes, scaled to the lanes that hold a sample
