@@ -327,31 +327,32 @@ __device__ __forceinline__ int block_level(const Params &p, const State<EXT> &s,
   const uint32_t k = s.m - 1u;
   const uint32_t fit = min(s.lim - s.n, p.last - 1u - k);  // >= 2: a block starts here
   const uint32_t top = min(min((uint32_t)__ffs((int)k) - 1u, p.bla_levels), 31u - (uint32_t)__clz((int)fit));
-  int lv = 0;
-  constexpr uint32_t PRE = 4;
+  uint32_t lv = 0;
+  bool run = true;
+  constexpr uint32_t PRE = 8, MORE = 4;
+  double r[PRE];
 #pragma unroll
-  for (uint32_t base = 1; base <= 1 + PRE; base += PRE) {
-    if (base < top) {
-      double r[PRE];
+  for (uint32_t q = 0; q < PRE; ++q)
+    r[q] = 1 + q < top ? __ldg(p.bla_r2 + (p.bla_off[1 + q] + (k >> (q + 2)))) : -1.0;
 #pragma unroll
-      for (uint32_t q = 0; q < PRE; ++q)
-        r[q] = base + q < top ? __ldg(p.bla_r2 + (p.bla_off[base + q] + (k >> (base + q + 1)))) : -1.0;
-      uint32_t pass = 0;
-#pragma unroll
-      for (uint32_t q = 0; q < PRE; ++q) pass |= (uint32_t)(d2 < r[q]) << q;
-      const int run = __ffs((int)~pass) - 1;  // bit PRE of ~pass is set: run <= PRE
-      lv += run;
-      if (run < (int)PRE) break;
-    }
+  for (uint32_t q = 0; q < PRE; ++q) {
+    run = run & (d2 < r[q]);
+    lv += run;
   }
-  if (lv == 2 * PRE) {
-    for (uint32_t i = 1 + 2 * PRE; i < top; ++i) {
-      if (!(d2 < __ldg(p.bla_r2 + (p.bla_off[i] + (k >> (i + 1)))))) break;
-      lv = (int)i;
+  if (run) {
+    for (uint32_t i = 1 + PRE; i < top && run; i += MORE) {
+#pragma unroll
+      for (uint32_t q = 0; q < MORE; ++q)
+        r[q] = i + q < top ? __ldg(p.bla_r2 + (p.bla_off[i + q] + (k >> (i + q + 1)))) : -1.0;
+#pragma unroll
+      for (uint32_t q = 0; q < MORE; ++q) {
+        run = run & (d2 < r[q]);
+        lv += run;
+      }
     }
   }
   at = k >> (lv + 1);
-  return lv;
+  return (int)lv;
 }
 
 // Contraction's own product of a lane's sample, kept in memory: only a sample iterated again
