@@ -1106,6 +1106,15 @@ fdc_status render_impl(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, const fdc
       ctx->blocks_per_sm[variant] = b > 0 ? b : 1;
     }
     dim3 grid(grid_blocks(ctx, ctx->blocks_per_sm[variant])), block(128);
+    // A launch of few samples spreads them over 12 warps an SM instead of filling the first
+    // warps: a warp of 32 lanes that diverge runs every lane's branches and waits for every
+    // lane's table loads (kernel ms at full warps / 4, 8, 12, 16 warps an SM: 64x36 shallow
+    // 0.418 / 0.343 0.333 0.329 0.351, 161x91 with blocks 1.12 / 1.09 0.95 0.85 0.94).
+    // Over the last three waves of the grid a warp reserves no slots ahead (401x227 without a
+    // table 1.15 -> 0.86 ms, 480x270 2.72 -> 2.49; an eighth of the queue where that is more).
+    const uint64_t spread = (uint64_t)ctx->sm_count * 12, lanes = (p.total + spread - 1) / spread;
+    p.idle_lanes = lanes < 32 ? (uint32_t)(32 - lanes) : 0;
+    p.tail = (uint32_t)std::max<uint64_t>(p.total / 8, 3ull * grid.x * block.x);
     void *args[] = {&p};
     CK(cudaLaunchKernel(fn, grid, block, args, 0, ctx->stream));
     CK(cudaGetLastError());

@@ -89,6 +89,8 @@ struct Params {
   uint64_t total;        // queue slots (tiles * 32)
   uint64_t deadline_ns;  // 0 = none
   uint32_t *timed_out;
+  uint32_t idle_lanes;  // lanes of each warp that take no sample (small launches)
+  uint32_t tail;        // slots left from which a warp takes only what its idle lanes need
   uint32_t defer;     // BLA lanes a warp gathers before it applies their blocks (warp_step)
   // Parameter-series start (series.rs:57-84, ordinary tiers): every sample starts at
   // iterate series_n from delta = sum_k b_k x^k, x = dc / rho; series_n = 0: none.
@@ -429,6 +431,14 @@ __device__ __forceinline__ Entry load_entry(const Params &p, uint32_t m) {
   return Entry{Z.x, Z.y, -1.0};
 }
 
+template <bool EXT, bool L>
+__device__ __forceinline__ void enter(const Params &p, State<EXT> &s) {
+  const Entry at = load_entry<L>(p, s.m);
+  s.Zr = at.zr;
+  s.Zi = at.zi;
+  if (L) s.r2a = at.r2a;
+}
+
 // A BLA block application (sample.rs:264-315): delta' = A delta + B dc, dz' = A dz + B.
 //
 // block_quick: the extended tier's application with its four normalisations (before and after,
@@ -509,6 +519,11 @@ __device__ __forceinline__ void apply_block(const Params &p, State<EXT> &s, int 
   const Block4 c = load_block(p.bla_coef + 2 * b);
   const double2 A = c.a, B = c.b;
   const uint32_t len = 2u << lv;
+  // the entry where the block ends, in flight together with its coefficients (a third of the
+  // chain of loads that a block waits for where few warps hide it)
+  s.m += len;
+  s.n += len;
+  enter<EXT, true>(p, s);
   if (__builtin_expect(!s.ct.times(A.x * A.x + A.y * A.y, 0) && s.gate != NO_GATE, 0))
     contraction_wide(s, product, A.x, A.y);
   if (!EXT && s.hold > 0) s.mu.multiply(A.x, A.y);
@@ -549,18 +564,8 @@ __device__ __forceinline__ void apply_block(const Params &p, State<EXT> &s, int 
     s.dc_r = s.ar * factor;
     s.dc_i = s.ai * factor;
   }
-  s.m += len;
-  s.n += len;
   s.blocks += 1;
   s.skipped += len;
-}
-
-template <bool EXT, bool L>
-__device__ __forceinline__ void enter(const Params &p, State<EXT> &s) {
-  const Entry at = load_entry<L>(p, s.m);
-  s.Zr = at.zr;
-  s.Zi = at.zi;
-  if (L) s.r2a = at.r2a;
 }
 
 // One ordinary step (sample.rs:331-380; number.rs:92-124): z = Z[m] + delta is carried
@@ -1009,16 +1014,16 @@ __device__ __forceinline__ bool step(const Params &p, State<EXT> &s, Result &res
 // consecutive slots (one tile), which the warp then hands to its idle lanes in order, so
 // one round trip to the head serves a tile instead of each lane as it finishes, and
 // neighbouring samples share a warp. Held slots start only as the warp's own lanes finish,
-// so over the last eighth of the queue a warp takes just the slots its idle lanes need:
-// there a long sample left waiting behind busy lanes would lengthen the launch's tail.
+// so over the last slots of the queue (`last`) a warp takes just the slots its idle lanes
+// need: there a long sample left waiting behind busy lanes would lengthen the launch's tail.
 // Every lane holds the same copy.
 struct Reservation {
   unsigned long long base = 0, end = 0;
-  bool tail = false;  // within the last eighth of the queue
+  bool tail = false;  // within the last slots of the queue
   // Slots for the `need` idle lanes (warp-uniform): false when the queue is spent;
   // otherwise the lanes of need with rank < count take first + rank.
-  __device__ __forceinline__ bool take(unsigned long long *queue, unsigned long long total, unsigned need,
-                                       unsigned lane, unsigned long long &first, unsigned &count) {
+  __device__ __forceinline__ bool take(unsigned long long *queue, unsigned long long total, unsigned long long last,
+                                       unsigned need, unsigned lane, unsigned long long &first, unsigned &count) {
     if (base >= end) {
       const unsigned long long grab = tail ? (unsigned long long)__popc(need) : 32ull;
       unsigned long long b = 0;
@@ -1027,7 +1032,7 @@ struct Reservation {
       if (b >= total) return false;
       base = b;
       end = b + grab < total ? b + grab : total;
-      tail = total - b <= total / 8;
+      tail = total - b <= last;
     }
     const unsigned long long left = end - base, want = (unsigned long long)__popc(need);
     count = (unsigned)(want < left ? want : left);
@@ -1056,7 +1061,6 @@ __device__ __forceinline__ bool warp_step(const Params &p, State<EXT> &s, Result
       if (T)  // sample.rs:267-281: the block start, for a later replay
         tr->snap(StripeSnap{s.m, s.n, s.xr, s.xi, s.delta_exp, s.scale, s.dc_r, s.dc_i, 0}, s.n + (2u << lv));
       apply_block<EXT, D>(p, s, lv, at, product);
-      enter<EXT, L>(p, s);
       upd = true;
     }
   }
@@ -1405,8 +1409,10 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(co
       tr->start(s.n);
     }
   };
+  const unsigned taking = FULL >> p.idle_lanes;
+  slots.tail = p.idle_lanes != 0;
   for (;;) {
-    unsigned need = __ballot_sync(FULL, !active);
+    unsigned need = __ballot_sync(FULL, !active) & taking;
     while (need && !exhausted) {
       if (p.deadline_ns) {
         uint64_t now = 0;
@@ -1420,11 +1426,11 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(co
       }
       unsigned long long base = 0;
       unsigned take = 0;
-      if (!slots.take(p.queue, p.total, need, lane, base, take)) {
+      if (!slots.take(p.queue, p.total, p.tail, need, lane, base, take)) {
         exhausted = true;
         break;
       }
-      if (!active) {
+      if (!active && ((need >> lane) & 1u)) {
         const unsigned rank = __popc(need & lt);
         const uint64_t slot = base + rank;
         if (rank < take) {
@@ -1449,7 +1455,7 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(co
           }
         }
       }
-      need = __ballot_sync(FULL, !active);
+      need = __ballot_sync(FULL, !active) & taking;
     }
     // the lanes step until one of them finishes
     const unsigned held = __ballot_sync(FULL, active);
@@ -1555,6 +1561,9 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks)
   uint32_t job = 0, counted = 0xffffffffu;
   Reservation slots;
   ExactProduct product;
+  // over the last three waves of the grid, or the last eighth of the queue, a warp reserves
+  // no slots ahead (as fdc_render's Params.tail)
+  const unsigned long long waves = 3ull * gridDim.x * blockDim.x, last = waves > total / 8 ? waves : total / 8;
   LaneCounters lc;
   lc.clear();
   // the BLA variants store a finished sample's raw state; encode_jobs_kernel computes the
@@ -1582,7 +1591,7 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks)
     while (need && !exhausted) {
       unsigned long long base = 0;
       unsigned take = 0;
-      if (!slots.take(queue, total, need, lane, base, take)) {
+      if (!slots.take(queue, total, last, need, lane, base, take)) {
         exhausted = true;
         break;
       }
