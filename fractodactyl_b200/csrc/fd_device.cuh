@@ -19,18 +19,19 @@ constexpr double RES2 = 1e-12 * 1e-12;        // RESOLVABLE^2, sample.rs:702-708
 constexpr double LN_2 = 0.6931471805599453;
 constexpr double TAU = 6.283185307179586;
 
-// crates/fd-fixed/src/lib.rs:32-42: 2^k as f64, exact where representable.
-__device__ __forceinline__ double exp2i(int64_t k) {
-  if (k > 1023) return __longlong_as_double(0x7ff0000000000000ll);
-  if (k >= -1022) return __longlong_as_double((long long)((uint64_t)(k + 1023) << 52));
-  if (k >= -1074) return __longlong_as_double((long long)(1ull << (k + 1074)));
-  return 0.0;
+// crates/fd-fixed/src/lib.rs:32-42: 2^k as f64, exact where representable (infinite from
+// 1024 up, 0 below -1074). Below the normal range as a product of two normal powers, whose
+// rounding is exact down to 2^-1074 and gives 0 from 2^-1075 down: a few instructions where
+// this is inlined, which its many uses in the kernels' rare paths need (instruction
+// fetch stalls the deep views).
+__device__ __forceinline__ double exp2i(int k) {
+  if ((unsigned)(k + 1022) <= 2046u) return __hiloint2double((k + 1023) << 20, 0);
+  if (k > 0) return __longlong_as_double(0x7ff0000000000000ll);
+  return 0x1p-1022 * __hiloint2double((max(k + 1022, -1022) + 1023) << 20, 0);
 }
 
-// The same for 32-bit exponents: one range test on the common path.
-__device__ __forceinline__ double exp2i(int k) {
-  if ((unsigned)(k + 1022) <= 2045u) return __hiloint2double((k + 1023) << 20, 0);
-  return exp2i((int64_t)k);
+__device__ __forceinline__ double exp2i(int64_t k) {
+  return exp2i((int)(k > 4000 ? 4000 : (k < -4000 ? -4000 : k)));
 }
 
 // Rust f64::max / f64::min ignore a NaN operand, as fmax/fmin do.
