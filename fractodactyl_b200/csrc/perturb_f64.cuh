@@ -444,63 +444,91 @@ __device__ __forceinline__ void enter(const Params &p, State<EXT> &s) {
 // block_quick: the extended tier's application with its four normalisations (before and after,
 // of delta and derivative) folded into one of each result. Scaling by a power of two is
 // exact and a normalised value does not depend on how it was scaled before, so the steps
-// around the block can be left out wherever no product counts that leaves binary64's
-// normal range, in this scaling or in the normalised one: the inputs in [2^-500, 2^100) (a
-// rebase near a nucleus leaves a mantissa down to 1e-145 for a few iterations), every part
-// of the results in [2^-600, 2^500) (a product below binary64's normal range in either
-// scaling then vanishes in the sum, and an overflow in either shows in one part at least),
-// and where dc or 1 is scaled below 2^-900, B's terms 80 binades below the results.
-// False, with nothing changed, for any other block (a zero part among them) and for a
-// mantissa so close to 2 that floor(log2) rounds up; apply_block then runs the full steps.
+// around the block can be left out wherever nothing that counts leaves binary64's normal
+// range in this scaling or in the normalised one. block_fits asks that of each result (high
+// words, 2^20 a binade): the input normal; the result's parts in [2^-951, 2^950), within
+// 2^900 of each other and of the input (its normalised value then lies within 2^900 of 1), so
+// that a product too small for binary64 vanishes in the sum and one too large shows in a
+// part; dc and the derivative's 1 less than 2^900 times the input, so that neither scaling
+// overflows; and b times an error of 2^-1055 in them, whose scaling may underflow, 80
+// binades below the result in both scalings. False, with nothing changed, for
+// any other block (a zero part among them) and for a mantissa so close to 2 that
+// floor(log2) rounds up; apply_block then runs the full steps.
 // Before, the normalisations were half of a block's instructions: with the level search's
 // conditions folded into one limit, 15.1 -> 13.1 warp instructions per executed operation and
 // 28.3 -> 25.4 ms a call on the 1920x1080 frame at a 1e-100 nucleus.
 __device__ __forceinline__ uint32_t magnitude_hi(double a) { return (uint32_t)__double2hiint(a) & 0x7fffffffu; }
 __device__ __forceinline__ double pow2(int k) { return __hiloint2double((1023 + k) << 20, 0); }  // -1022 <= k <= 1023
 
+__device__ __forceinline__ bool block_fits(uint32_t in, uint32_t top, uint32_t low, uint32_t b) {
+  constexpr uint32_t ONE = 1023u << 20, FAR = 900u << 20;
+  return (in - (40u << 20) < (2000u << 20)) & (low >= (72u << 20)) & (top < (1973u << 20)) & (top - low <= FAR) &
+         ((int)(top - in) <= (int)FAR) & ((int)(in - low) <= (int)FAR) & (b + max(in, ONE) <= low + (1998u << 20)) &
+         ((top & 0xfffffu) != 0xfffffu);
+}
+
 template <bool D>
 __device__ __forceinline__ bool block_quick(State<true> &s, double2 A, double2 B) {
-  constexpr uint32_t ONE = 1023u << 20;
-  const uint32_t xh = max(magnitude_hi(s.xr), magnitude_hi(s.xi));
-  uint32_t lo = xh, hi = xh;
-  if (D) {
-    const uint32_t dh = max(magnitude_hi(s.dr), magnitude_hi(s.di));
-    lo = min(lo, dh);
-    hi = max(hi, dh);
-  }
-  bool ok = lo >= ONE - (500u << 20) && hi < ONE + (100u << 20);
+  const uint32_t bh = max(magnitude_hi(B.x), magnitude_hi(B.y));
   const double xr = A.x * s.xr - A.y * s.xi + B.x * s.dc_r - B.y * s.dc_i;
   const double xi = A.x * s.xi + A.y * s.xr + B.x * s.dc_i + B.y * s.dc_r;
-  const uint32_t xrh = magnitude_hi(xr), xih = magnitude_hi(xi), rx = max(xrh, xih);
-  const uint32_t low = min(xrh, xih);
-  ok &= low >= ONE - (600u << 20) && rx < ONE + (500u << 20) && (rx & 0xfffffu) != 0xfffffu;
-  const int off = s.offset_exp - s.delta_exp;  // dc's parts are below 2^20 2^off
-  if (off < -900) ok &= (int)(max(magnitude_hi(B.x), magnitude_hi(B.y)) >> 20) + off + 100 <= (int)(low >> 20);
+  const uint32_t xrh = magnitude_hi(xr), xih = magnitude_hi(xi), top = max(xrh, xih);
+  const uint32_t xh = max(magnitude_hi(s.xr), magnitude_hi(s.xi));
+  bool ok = block_fits(xh, top, min(xrh, xih), bh) & (s.offset_exp - s.delta_exp + 1043 - (int)(xh >> 20) <= 900);
   if (D) {
     const double dr = A.x * s.dr - A.y * s.di + B.x * s.inverse;
     const double di = A.x * s.di + A.y * s.dr + B.y * s.inverse;
-    const uint32_t drh = magnitude_hi(dr), dih = magnitude_hi(di), rd = max(drh, dih);
-    const uint32_t dlow = min(drh, dih);
-    ok &= dlow >= ONE - (600u << 20) && rd < ONE + (500u << 20) && (rd & 0xfffffu) != 0xfffffu;
-    if (s.derivative_exp > 900)
-      ok &= (int64_t)(max(magnitude_hi(B.x), magnitude_hi(B.y)) >> 20) - s.derivative_exp + 80 <= (int64_t)(dlow >> 20);
+    const uint32_t drh = magnitude_hi(dr), dih = magnitude_hi(di), dtop = max(drh, dih);
+    const uint32_t dh = max(magnitude_hi(s.dr), magnitude_hi(s.di));
+    ok &= block_fits(dh, dtop, min(drh, dih), bh) & (__double2hiint(s.inverse) - (int)dh <= (int)(900u << 20));
     if (!ok) return false;
-    const int k = (int)(rd >> 20) - 1023;
+    const int k = (int)(dtop >> 20) - 1023;
     const double f = pow2(-k);
     s.dr = dr * f;
     s.di = di * f;
     s.derivative_exp += k;
-    s.inverse = s.derivative_exp >= -1023 && s.derivative_exp <= 1022 ? pow2(-(int)s.derivative_exp)
-                                                                      : exp2i(-s.derivative_exp);
+    s.inverse = exp2i(-s.derivative_exp);
   } else if (!ok) {
     return false;
   }
-  const int k = min((int)(rx >> 20) - 1023, -s.delta_exp);  // the exponent stays at or below 0
+  const int k = min((int)(top >> 20) - 1023, -s.delta_exp);  // the exponent stays at or below 0
   const double f = pow2(-k);
   s.xr = xr * f;
   s.xi = xi * f;
   s.delta_exp += k;
   return true;
+}
+
+// The extended tier's application in full, out of line: no block of ordinary views takes it,
+// and inlined its four normalisations stretched the loop's code.
+struct BlockTerms {
+  double xr, xi, dr, di, inverse;
+  int64_t derivative_exp;
+  int32_t delta_exp;
+};
+
+template <bool D>
+static __device__ __noinline__ BlockTerms block_full(BlockTerms s, double2 A, double2 B, double ar, double ai,
+                                                     int32_t offset_exp) {
+  normalise(s.xr, s.xi, s.delta_exp, 0);
+  if (D) {
+    normalise(s.dr, s.di, s.derivative_exp, INT64_MAX / 4);
+    s.inverse = exp2i(-s.derivative_exp);
+    const double t = A.x * s.dr - A.y * s.di + B.x * s.inverse;
+    s.di = A.x * s.di + A.y * s.dr + B.y * s.inverse;
+    s.dr = t;
+  }
+  const double factor = exp2i(offset_exp - s.delta_exp);
+  const double dc_r = ar * factor, dc_i = ai * factor;
+  const double t = A.x * s.xr - A.y * s.xi + B.x * dc_r - B.y * dc_i;
+  s.xi = A.x * s.xi + A.y * s.xr + B.x * dc_i + B.y * dc_r;
+  s.xr = t;
+  normalise(s.xr, s.xi, s.delta_exp, 0);
+  if (D) {
+    normalise(s.dr, s.di, s.derivative_exp, INT64_MAX / 4);
+    s.inverse = exp2i(-s.derivative_exp);
+  }
+  return s;
 }
 
 template <bool EXT, bool D>
@@ -527,22 +555,24 @@ __device__ __forceinline__ void apply_block(const Params &p, State<EXT> &s, int 
   if (__builtin_expect(!s.ct.times(A.x * A.x + A.y * A.y, 0) && s.gate != NO_GATE, 0))
     contraction_wide(s, product, A.x, A.y);
   if (!EXT && s.hold > 0) s.mu.multiply(A.x, A.y);
-  if (!BlockQuick<EXT, D>::run(s, A, B)) {
-    if (EXT) {
-      normalise(s.xr, s.xi, s.delta_exp, 0);
-      if (D) {
-        normalise(s.dr, s.di, s.derivative_exp, INT64_MAX / 4);
-        s.inverse = exp2i(-s.derivative_exp);
-      }
-      const double factor = exp2i(s.offset_exp - s.delta_exp);
-      s.dc_r = s.ar * factor;
-      s.dc_i = s.ai * factor;
+  if (EXT) {
+    if (!BlockQuick<EXT, D>::run(s, A, B)) {
+      const BlockTerms t = block_full<D>(BlockTerms{s.xr, s.xi, s.dr, s.di, s.inverse, s.derivative_exp, s.delta_exp}, A,
+                                         B, s.ar, s.ai, s.offset_exp);
+      s.xr = t.xr;
+      s.xi = t.xi;
+      s.dr = t.dr;
+      s.di = t.di;
+      s.inverse = t.inverse;
+      s.derivative_exp = t.derivative_exp;
+      s.delta_exp = t.delta_exp;
     }
+  } else {
     if (D) {
       double t = A.x * s.dr - A.y * s.di + B.x * s.inverse;
       s.di = A.x * s.di + A.y * s.dr + B.y * s.inverse;
       s.dr = t;
-      if (!EXT && (p.flags & F_SHIFT)) {
+      if (p.flags & F_SHIFT) {
         double2 ab = __ldg(p.bla_ab + b);
         s.shift += (ab.x * sqrt(s.xr * s.xr + s.xi * s.xi) + ab.y * s.adc) / sqrt(s.dr * s.dr + s.di * s.di);
       }
@@ -550,13 +580,6 @@ __device__ __forceinline__ void apply_block(const Params &p, State<EXT> &s, int 
     double t = A.x * s.xr - A.y * s.xi + B.x * s.dc_r - B.y * s.dc_i;
     s.xi = A.x * s.xi + A.y * s.xr + B.x * s.dc_i + B.y * s.dc_r;
     s.xr = t;
-    if (EXT) {
-      normalise(s.xr, s.xi, s.delta_exp, 0);
-      if (D) {
-        normalise(s.dr, s.di, s.derivative_exp, INT64_MAX / 4);
-        s.inverse = exp2i(-s.derivative_exp);
-      }
-    }
   }
   if (EXT) {
     s.scale = exp2i(s.delta_exp);
@@ -1043,19 +1066,32 @@ struct Reservation {
 };
 
 // One iteration for the lanes of a warp that hold a sample (`held`, warp-uniform; every lane
-// of the warp calls it). A lane whose next operation is a BLA block waits until thr lanes
-// wait or no lane steps plainly; the waiting lanes then apply their blocks together. The
-// warp runs the block path for many lanes at a time instead of for one or two lanes on
-// nearly every iteration, and each lane's own sequence of operations is unchanged.
+// of the warp calls it). A lane whose next operation is a BLA block (s.on), or that has its
+// outcome (done), waits until thr lanes wait or no lane steps plainly; the waiting lanes
+// then apply their blocks together. The warp runs the block path for many lanes at a time
+// instead of for one or two lanes on nearly every iteration, and each lane's own sequence of
+// operations is unchanged. Returns the lanes that are done where the warp should look
+// (warp-uniform): with BLA only when the waiting lanes have their turn, one vote a step.
 template <bool EXT, bool D, bool L, bool B = false, bool T = false>
-__device__ __forceinline__ bool warp_step(const Params &p, State<EXT> &s, Result &res, bool active, unsigned held,
-                                          uint32_t thr, ExactProduct &product, StripeTrace *tr = nullptr) {
-  bool upd = active;
-  if (L) upd = active && !s.on;
+__device__ __forceinline__ unsigned warp_step(const Params &p, State<EXT> &s, Result &res, bool active, bool &done,
+                                              unsigned held, uint32_t thr, ExactProduct &product,
+                                              StripeTrace *tr = nullptr) {
+  const unsigned FULL = 0xffffffffu;
+  if (!L) {
+    if (active) {
+      plain_update<EXT, D, L, B>(p, s);
+      done = post<EXT, D, L, B, T>(p, s, res, product, tr);
+    }
+    return __ballot_sync(FULL, done);
+  }
+  const bool wait = s.on | done;  // neither in a lane without a sample
+  bool upd = active && !wait;
   if (upd) plain_update<EXT, D, L, B>(p, s);
-  if (L) {
-    const unsigned waiting = __ballot_sync(0xffffffffu, active && s.on);
-    if (((uint32_t)__popc(waiting) >= thr || waiting == held) && active && s.on) {
+  const unsigned waiting = __ballot_sync(FULL, wait);
+  unsigned ended = 0;
+  if ((uint32_t)__popc(waiting) >= thr || waiting == held) {
+    ended = __ballot_sync(FULL, done);
+    if (wait && !done) {
       uint32_t at;
       const int lv = block_level(p, s, at);
       if (T)  // sample.rs:267-281: the block start, for a later replay
@@ -1064,7 +1100,8 @@ __device__ __forceinline__ bool warp_step(const Params &p, State<EXT> &s, Result
       upd = true;
     }
   }
-  return upd && post<EXT, D, L, B, T>(p, s, res, product, tr);
+  if (upd) done = post<EXT, D, L, B, T>(p, s, res, product, tr);
+  return ended;
 }
 
 // The threshold of warp_step: defer of 32 lanes, scaled to the lanes that hold a sample
@@ -1113,10 +1150,10 @@ __device__ __forceinline__ void start_sample(const Params &p, State<EXT> &s, boo
 
 template <bool EXT, bool D, bool L, bool S = false, bool B = false>
 __device__ __forceinline__ int init(const Params &p, uint64_t slot, State<EXT> &s, Result &res) {
-  uint64_t tile = slot >> 5;
+  uint32_t tile = (uint32_t)(slot >> 5);  // fewer than 2^31 samples
   if (p.tile_order) tile = __ldg(p.tile_order + tile);  // queue position -> row-major tile
   uint32_t w = (uint32_t)slot & 31u;
-  uint32_t tx = (uint32_t)(tile % p.tiles_x), ty = (uint32_t)(tile / p.tiles_x);
+  const uint32_t ty = tile / p.tiles_x, tx = tile - ty * p.tiles_x;
   uint32_t ii = (tx << p.tile_shift) + (w & ((1u << p.tile_shift) - 1u));
   uint32_t jj = ty * (32u >> p.tile_shift) + (w >> p.tile_shift);
   if (ii >= p.cols || jj >= p.rows) return 0;
@@ -1368,9 +1405,10 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(co
   const unsigned lt = (1u << lane) - 1u;
   State<EXT> s;
   Result res;
-  bool active = false, exhausted = false;
+  bool active = false, done = false, exhausted = false;
   Reservation slots;
   ExactProduct product;
+  s.on = false;
   TraceSlot<T> trace;
   StripeTrace *tr = trace.get();
   uint64_t t0 = p.deadline_ns ? globaltimer() : 0;
@@ -1457,37 +1495,35 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(co
       }
       need = __ballot_sync(FULL, !active) & taking;
     }
-    // the lanes step until one of them finishes
+    // the lanes step until some of them have an outcome
     const unsigned held = __ballot_sync(FULL, active);
     if (!held) break;
     const uint32_t thr = threshold(held, p.defer);
     unsigned ended = 0;
     do {
-      bool done = warp_step<EXT, D, L, B, T>(p, s, res, active, held, thr, product, tr);
-      if (__builtin_expect(done, 0)) {
-        if (S && bias > 0 && res.kind == 2) {
-          retry();
-          done = false;
-        } else if (res.kind == 3) {  // once more, for Contraction's own product
-          start_sample<EXT, D, L, B>(p, s, false, S);
-          if (S) {
-            s.blocks = blocks0;
-            s.skipped = skipped0;
-          }
-          if (T) {
-            tr->begin();
-            tr->start(s.n);
-          }
-          s.ct.take_exact();
-          product.reset();
-          done = false;
-        }
-      }
-      ended = __ballot_sync(FULL, done);
+      ended = warp_step<EXT, D, L, B, T>(p, s, res, active, done, held, thr, product, tr);
     } while (!ended);
     if ((ended >> lane) & 1u) {
-      finish(s.idx, res, s.blocks, s.skipped, s.shift);
-      active = false;
+      done = false;
+      if (S && bias > 0 && res.kind == 2) {
+        retry();
+      } else if (res.kind == 3) {  // once more, for Contraction's own product
+        start_sample<EXT, D, L, B>(p, s, false, S);
+        if (S) {
+          s.blocks = blocks0;
+          s.skipped = skipped0;
+        }
+        if (T) {
+          tr->begin();
+          tr->start(s.n);
+        }
+        s.ct.take_exact();
+        product.reset();
+      } else {
+        finish(s.idx, res, s.blocks, s.skipped, s.shift);
+        active = false;
+        s.on = false;
+      }
     }
   }
   // warp reduction of the counters, one atomic per warp
@@ -1557,10 +1593,11 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks)
   const unsigned lt = (1u << lane) - 1u;
   State<EXT> s;
   Result res;
-  bool active = false, exhausted = false;
+  bool active = false, done = false, exhausted = false;
   uint32_t job = 0, counted = 0xffffffffu;
   Reservation slots;
   ExactProduct product;
+  s.on = false;
   // over the last three waves of the grid, or the last eighth of the queue, a warp reserves
   // no slots ahead (as fdc_render's Params.tail)
   const unsigned long long waves = 3ull * gridDim.x * blockDim.x, last = waves > total / 8 ? waves : total / 8;
@@ -1617,18 +1654,19 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks)
     const Params &p = jobs[job];
     unsigned ended = 0;
     do {
-      bool done = warp_step<EXT, D, L>(p, s, res, active, held, thr, product);
-      if (__builtin_expect(done && res.kind == 3, 0)) {  // once more, for Contraction's own product
+      ended = warp_step<EXT, D, L>(p, s, res, active, done, held, thr, product);
+    } while (!ended);
+    if ((ended >> lane) & 1u) {
+      done = false;
+      if (res.kind == 3) {  // once more, for Contraction's own product
         start_sample<EXT, D, L, false>(p, s, false, false);
         s.ct.take_exact();
         product.reset();
-        done = false;
+      } else {
+        finish(p, s.idx, res, s.blocks, s.skipped);
+        active = false;
+        s.on = false;
       }
-      ended = __ballot_sync(FULL, done);
-    } while (!ended);
-    if ((ended >> lane) & 1u) {
-      finish(p, s.idx, res, s.blocks, s.skipped);
-      active = false;
     }
   }
   if (counted != 0xffffffffu) lc.flush(per_job + counted);
