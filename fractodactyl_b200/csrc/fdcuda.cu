@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <condition_variable>
 #include <map>
 #include <memory>
@@ -95,6 +96,7 @@ struct fdc_ctx {
   // next upload of the same size: a film or a service re-uploading per frame allocates
   // once. Stream-ordered: every user runs on `stream`. Freed by fdc_close.
   std::multimap<size_t, void *> pool;
+  char *small = nullptr;  // pinned staging of a small render's columns and counters
   // pinned staging for large host<->device copies: two chunk slots, each with the event
   // of the last transfer that used it
   char *pinned = nullptr;
@@ -381,12 +383,16 @@ void free_batch(fdc_batch *b) {
   delete b;
 }
 
+// A render whose columns fit in SMALL bytes brings them back in one copy to pinned memory.
+constexpr size_t SMALL = 1u << 20;
+
 fdc_status open_resources(fdc_ctx *ctx) {
   CK(cudaSetDevice(ctx->device));
   CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
   CK(cudaEventCreate(&ctx->ev0));
   CK(cudaEventCreate(&ctx->ev1));
   CK(cudaMalloc(&ctx->scratch, sizeof(Scratch)));
+  CK(cudaHostAlloc((void **)&ctx->small, SMALL + sizeof(Scratch), cudaHostAllocDefault));
   CK(cudaEventCreateWithFlags(&ctx->slot_ev[0], cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&ctx->slot_ev[1], cudaEventDisableTiming));
   return FDC_OK;
@@ -424,34 +430,35 @@ class CopyPool {
     go_.notify_all();
     for (auto &t : threads_) t.join();
   }
+  size_t parts() const { return threads_.size() + 1; }
   void copy(void *dst, const void *src, size_t bytes) {
-    const size_t workers = threads_.size();
-    if (workers == 0 || bytes < (256u << 10)) {
+    if (threads_.empty() || bytes < (256u << 10)) {
       std::memcpy(dst, src, bytes);
       return;
     }
+    const size_t part = ((bytes / parts()) + 63) & ~(size_t)63;
+    each([=](size_t k) {
+      const size_t a = std::min(bytes, k * part), b = std::min(bytes, a + part);
+      if (b > a) std::memcpy((char *)dst + a, (const char *)src + a, b - a);
+    });
+  }
+  // work(k) for every part k < parts(), this thread's the last
+  template <class F>
+  void each(const F &work) {
     {
       std::lock_guard<std::mutex> l(m_);
-      dst_ = (char *)dst;
-      src_ = (const char *)src;
-      bytes_ = bytes;
-      part_ = ((bytes / (workers + 1)) + 63) & ~(size_t)63;
-      pending_ = workers;
+      work_ = &work;
+      call_ = [](const void *w, size_t k) { (*(const F *)w)(k); };
+      pending_ = threads_.size();
       ++gen_;
     }
     go_.notify_all();
-    piece(workers);
+    work(threads_.size());
     std::unique_lock<std::mutex> l(m_);
     done_.wait(l, [&] { return pending_ == 0; });
   }
 
  private:
-  // part k of the current copy; its fields were set under the lock before the workers
-  // were woken and stay until every part is done
-  void piece(size_t k) {
-    const size_t a = std::min(bytes_, k * part_), b = std::min(bytes_, a + part_);
-    if (b > a) std::memcpy(dst_ + a, src_ + a, b - a);
-  }
   void run(unsigned id) {
     uint64_t seen = 0;
     for (;;) {
@@ -461,7 +468,7 @@ class CopyPool {
         if (stop_) return;
         seen = gen_;
       }
-      piece(id);
+      call_(work_, id);  // set under the lock before the wake-up, and kept until every part is done
       std::lock_guard<std::mutex> l(m_);
       if (--pending_ == 0) done_.notify_one();
     }
@@ -472,16 +479,18 @@ class CopyPool {
   uint64_t gen_ = 0;
   size_t pending_ = 0;
   bool stop_ = false;
-  char *dst_ = nullptr;
-  const char *src_ = nullptr;
-  size_t bytes_ = 0, part_ = 0;
+  const void *work_ = nullptr;
+  void (*call_)(const void *, size_t) = nullptr;
 };
 
+void ensure_copier(fdc_ctx *ctx) {
+  if (ctx->copier) return;
+  const unsigned hw = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
+  ctx->copier = std::make_unique<CopyPool>(hw - 1);
+}
+
 cudaError_t ensure_pinned(fdc_ctx *ctx) {
-  if (!ctx->copier) {
-    const unsigned hw = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
-    ctx->copier = std::make_unique<CopyPool>(hw - 1);
-  }
+  ensure_copier(ctx);
   if (ctx->pinned) return cudaSuccess;
   return cudaHostAlloc((void **)&ctx->pinned, 2 * CHUNK, cudaHostAllocDefault);
 }
@@ -525,6 +534,50 @@ cudaError_t download(fdc_ctx *ctx, void *dst, const void *src, size_t bytes) {
   return e;
 }
 
+// max over n pairs of hypot(x, y), as a loop from 0 over std::hypot gives it (a NaN pair
+// passed over): the largest x^2 + y^2 first, then hypot of the pairs within 1e-14 of it,
+// where the squares stay in range (a pair further below has a smaller hypot, whose error is
+// within an ulp). hypot over every offset of a jittered frame took longer than its
+// transfer: 2880x1620 samples 17 -> 1 ms on 8 threads.
+double largest_hypot(fdc_ctx *ctx, const double *xy, uint64_t n) {
+  const auto full = [&]() {
+    double h = 0.0;
+    for (uint64_t k = 0; k < 2 * n; k += 2) h = std::max(h, std::hypot(xy[k], xy[k + 1]));
+    return h;
+  };
+  if (n < 4096) return full();
+  ensure_copier(ctx);
+  const size_t parts = ctx->copier->parts();
+  const uint64_t part = (n + parts - 1) / parts;
+  double top[8 * 8] = {}, best[8 * 8] = {};  // a cache line a part, of at most 8 (ensure_copier)
+  ctx->copier->each([&](size_t p) {
+    const uint64_t a = std::min<uint64_t>(n, p * part), b = std::min<uint64_t>(n, a + part);
+    double m = 0.0;
+    bool odd = false;
+    for (uint64_t k = 2 * a; k < 2 * b; k += 2) {
+      const double q = xy[k] * xy[k] + xy[k + 1] * xy[k + 1];
+      odd |= !(q < 1e300);
+      m = q > m ? q : m;
+    }
+    top[8 * p] = odd ? std::numeric_limits<double>::infinity() : m;
+  });
+  double m = 0.0;
+  for (size_t p = 0; p < parts; ++p) m = std::max(m, top[8 * p]);
+  if (!(m > 1e-280 && m < 1e300)) return full();
+  const double near = m * (1.0 - 1e-14);
+  ctx->copier->each([&](size_t p) {
+    if (top[8 * p] < near) return;
+    const uint64_t a = std::min<uint64_t>(n, p * part), b = std::min<uint64_t>(n, a + part);
+    double h = 0.0;
+    for (uint64_t k = 2 * a; k < 2 * b; k += 2)
+      if (xy[k] * xy[k] + xy[k + 1] * xy[k + 1] >= near) h = std::max(h, std::hypot(xy[k], xy[k + 1]));
+    best[8 * p] = h;
+  });
+  double h = 0.0;
+  for (size_t p = 0; p < parts; ++p) h = std::max(h, best[8 * p]);
+  return h;
+}
+
 // Validate a job against its orbit (the refusals of render_bla, grid.rs:378-413) and fill
 // the per-job part of the kernel parameters (everything but outputs, queue, counters).
 fdc_status prepare(fdc_ctx *ctx, const OrbitDev &o, const fdc_job &j, fdk::Params &p, uint32_t &first,
@@ -556,11 +609,7 @@ fdc_status prepare(fdc_ctx *ctx, const OrbitDev &o, const fdc_job &j, fdk::Param
   // Largest unit offset: the grid's corner (grid.rs:428-444), or the supplied offsets'.
   auto largest_offset = [&]() {
     double half = std::hypot((double)j.nx / 2.0, (double)j.ny / 2.0);
-    if (j.offsets) {
-      half = 0.0;
-      const uint64_t lo = 2ull * first * j.nx, hi = 2ull * (first + rows) * j.nx;
-      for (uint64_t k = lo; k < hi; k += 2) half = std::max(half, std::hypot(j.offsets[k], j.offsets[k + 1]));
-    }
+    if (j.offsets) half = largest_hypot(ctx, j.offsets + 2ull * first * j.nx, (uint64_t)rows * j.nx);
     return half;
   };
   if (series) {  // Series::render_masked's refusals (grid.rs:341-366)
@@ -683,6 +732,7 @@ void fdc_close(fdc_ctx *ctx) {
   ctx->orders.clear();
   ctx->copier.reset();
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
+  if (ctx->small) cudaFreeHost(ctx->small);
   for (auto &ev : ctx->slot_ev)
     if (ev) cudaEventDestroy(ev);
   cudaFree(ctx->scratch);
@@ -1021,13 +1071,20 @@ fdc_status render_impl(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, const fdc
   if (encode_later)
     for (int c : {0, 1, 5, 6, 7, 8}) scratch[c] = cols[c].host == nullptr;
   const uint64_t scratch_rows = (uint64_t)rows * (dev_out ? j.nx : p.cols);
+  // the staged columns, those to be copied back first, then the scratch: one region
   size_t need = 0;
   size_t offs[NCOL + 2];
   for (int c = 0; c < NCOL; ++c) {
     offs[c] = need;
-    if (scratch[c]) need += (scratch_rows * cols[c].width + 255) & ~(size_t)255;
-    else if (cols[c].host && !dev_out) need += (n_rows * cols[c].width + 255) & ~(size_t)255;
+    if (cols[c].host && !dev_out) need += (n_rows * cols[c].width + 255) & ~(size_t)255;
   }
+  const size_t back = need;
+  for (int c = 0; c < NCOL; ++c)
+    if (scratch[c]) {
+      offs[c] = need;
+      need += (scratch_rows * cols[c].width + 255) & ~(size_t)255;
+    }
+  const size_t staged = need;
   offs[NCOL] = need;  // mask
   if (j.mask) need += (n_rows + 255) & ~(size_t)255;
   offs[NCOL + 1] = need;  // offsets
@@ -1072,12 +1129,11 @@ fdc_status render_impl(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, const fdc
                    cudaMemcpyHostToDevice));
   }
   // Samples that are never reached keep zeroed columns and status 0.
-  for (int c = 0; c < NCOL; ++c) {
-    if (!dptr[c]) continue;
+  if (staged) CK(cudaMemsetAsync(stage, 0, staged, ctx->stream));
+  for (int c = 0; dev_out && c < NCOL; ++c) {
+    if (!dptr[c] || scratch[c]) continue;
     const size_t w = cols[c].width;
-    if (scratch[c])
-      CK(cudaMemsetAsync(dptr[c], 0, scratch_rows * w, ctx->stream));
-    else if (!dev_out || full)
+    if (full)
       CK(cudaMemsetAsync(dptr[c], 0, n_rows * w, ctx->stream));
     else
       CK(cudaMemset2DAsync(dptr[c], j.nx * w, 0, p.cols * w, rows, ctx->stream));
@@ -1125,7 +1181,14 @@ fdc_status render_impl(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, const fdc
     }
   }
   CK(cudaEventRecord(ctx->ev1, ctx->stream));
-  if (!dev_out) {
+  // Small frames come back in one copy to pinned memory and are spread from there (a copy to
+  // pageable memory for each column waited for each: 7 of them and as many clears took a
+  // quarter of a 64x36 call); large ones column by column through the pinned chunks.
+  const bool merged = back > 0 && back <= SMALL;
+  Scratch &sc = *(Scratch *)(ctx->small + SMALL);
+  if (merged) {
+    CK(cudaMemcpyAsync(ctx->small, stage, back, cudaMemcpyDeviceToHost, ctx->stream));
+  } else if (!dev_out) {
     for (int c = 0; c < NCOL; ++c)
       if (cols[c].host) {
         const size_t w = cols[c].width;
@@ -1133,9 +1196,17 @@ fdc_status render_impl(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, const fdc
                        cudaMemcpyDeviceToHost));
       }
   }
-  Scratch sc;
   CK(cudaMemcpyAsync(&sc, ctx->scratch, sizeof sc, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
+  for (int c = 0; merged && c < NCOL; ++c) {
+    if (!cols[c].host) continue;
+    const size_t w = cols[c].width, row = p.cols * w;
+    char *to = (char *)cols[c].host + origin * w;
+    const char *from = ctx->small + offs[c];
+    if (full) std::memcpy(to, from, row * rows);
+    else
+      for (uint32_t r = 0; r < rows; ++r) std::memcpy(to + (size_t)r * j.nx * w, from + r * row, row);
+  }
   if (counters) {
     float ms = 0;
     CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
