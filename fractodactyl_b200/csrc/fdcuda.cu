@@ -1171,6 +1171,13 @@ fdc_status render_impl(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, const fdc
     const uint64_t spread = (uint64_t)ctx->sm_count * 12, lanes = (p.total + spread - 1) / spread;
     p.idle_lanes = lanes < 32 ? (uint32_t)(32 - lanes) : 0;
     p.tail = (uint32_t)std::max<uint64_t>(p.total / 8, 3ull * grid.x * block.x);
+    const size_t trace_bytes = stripe ? sizeof(fdk::StripeTrace) * grid.x * block.x : 0;
+    if (stripe) {
+      p.stripe_traces = (fdk::StripeTrace *)pool_get(ctx, trace_bytes);
+      if (!p.stripe_traces) return fail(ctx, FDC_DEVICE_ERROR, "device memory for the stripe recorders");
+    }
+    // back to the pool in stream order: its next user runs after this kernel
+    pool_put(ctx, p.stripe_traces, trace_bytes);
     void *args[] = {&p};
     CK(cudaLaunchKernel(fn, grid, block, args, 0, ctx->stream));
     CK(cudaGetLastError());

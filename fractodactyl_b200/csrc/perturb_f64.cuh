@@ -38,6 +38,8 @@ struct Counters {
   unsigned long long pad;
 };
 
+struct StripeTrace;
+
 // Everything one launch needs; passed by value (kernel parameter space).
 struct Params {
   const double2 *__restrict__ orbit;  // Z_0..Z_last, interleaved re/im
@@ -106,6 +108,7 @@ struct Params {
   float *stripe_out;
   uint32_t stripe_window;
   double stripe_freq;
+  StripeTrace *stripe_traces;  // a recorder for every thread of the grid
 };
 
 constexpr double SAFE = 1.0 + 8.0 * U;  // sample.rs:56
@@ -162,7 +165,10 @@ struct StripeSnap {
 
 // The Stripe column's recorder for one lane (stripe.rs:12-241): the last 128 iterates, the
 // last 8 block starts, and the escape the blocks found while a replay re-walks its window.
-// Only the stripe variants (T) hold one; it lives in local memory (~2.6 KB per lane).
+// Only the stripe variants (T) hold one. It lies in one piece in global memory (2.6 KB a lane,
+// 200 MB a grid): the iterates a lane records one after the other fill whole sectors. In local
+// memory, which interleaves a warp's lanes word by word, lanes at different iterates wrote
+// four sectors an iterate with four bytes each.
 struct StripeTrace {
   static constexpr uint32_t RING = 128, SNAPS = 8;
   double2 ring[RING];
@@ -172,12 +178,12 @@ struct StripeTrace {
   uint64_t first_at;
   uint64_t valid;
   uint32_t count;
-  float value;
+  uint64_t end_at;  // the iterate the outcome's window ends at (end), and z there
+  double end_r, end_i;
 
   __device__ __forceinline__ void begin() {  // stripe.rs:164-168
     valid = ~0ull;
     count = 0;
-    value = 0.0f;
   }
   __device__ __forceinline__ void start(uint64_t n) { valid = n + 1; }
   __device__ __forceinline__ void record(uint64_t n, double zr, double zi) { ring[n % RING] = make_double2(zr, zi); }
@@ -228,36 +234,53 @@ struct StripeTrace {
     }
     return 0.5 + 0.5 * s;
   }
-  // stripe.rs:206-240: the windows ending at z_n and z_{n-1}, interpolated by how far
-  // past the escape radius z_n landed
-  __device__ void finish(uint64_t n, double zr, double zi, double r2, uint32_t window, double k) {
+  __device__ __forceinline__ void end(uint64_t n, double zr, double zi) {
+    end_at = n;
+    end_r = zr;
+    end_i = zi;
+  }
+  // stripe.rs:206-240: the windows ending at z_n and z_{n-1}, interpolated by how far past the
+  // escape radius z_n landed, by a whole warp: each lane takes the term of one iterate, and
+  // all add them in the reference's order. One lane after the other for every finished
+  // sample, the terms (a hypot, two divisions or a sine each) were most of the kernel's work.
+  __device__ float average(unsigned lane, double r2, uint32_t window, double k) const {
+#if defined(__CUDA_ARCH__)
+    constexpr uint64_t LANES = 32;
+#else
+    constexpr uint64_t LANES = 1;  // host builds run a warp of one lane
+#endif
+    const uint64_t n = end_at, from = valid;
     const uint64_t lo = n > window ? n - window : 0;
     const uint64_t first_i = lo > 1 ? lo : 1;
     double now = 0.0, before = 0.0;
     uint32_t cn = 0, cb = 0;
-    for (uint64_t i = first_i; i <= n; ++i) {
-      if (i < valid) continue;
-      const double2 z = ring[i % RING];
-      const double t = term(z.x, z.y, k);
-      if (i > first_i || (first_i == 1 && n <= window)) {
-        now += t;
-        cn += 1;
+    for (uint64_t base = first_i; base <= n; base += LANES) {
+      const uint64_t mine = base + lane;
+      double own = 0.0;
+      if (mine <= n && mine >= from) {
+        const double2 z = ring[mine % RING];
+        own = term(z.x, z.y, k);
       }
-      if (i < n) {
-        before += t;
-        cb += 1;
+      for (uint64_t i = base; i < base + LANES && i <= n; ++i) {
+        const double t = __shfl_sync(0xffffffffu, own, (int)(i - base));
+        if (i < from) continue;
+        if (i > first_i || (first_i == 1 && n <= window)) {
+          now += t;
+          cn += 1;
+        }
+        if (i < n) {
+          before += t;
+          cb += 1;
+        }
       }
     }
-    if (cn == 0) {
-      value = 0.0f;
-      return;
-    }
+    if (cn == 0) return 0.0f;
     now /= (double)cn;
     before = cb > 0 ? before / (double)cb : now;
-    double frac = 1.0 - log2(log(zr * zr + zi * zi) / log(r2));
+    double frac = 1.0 - log2(log(end_r * end_r + end_i * end_i) / log(r2));
     if (frac < 0.0) frac = 0.0;  // f64::clamp keeps NaN
     if (frac > 1.0) frac = 1.0;
-    value = (float)(before * (1.0 - frac) + now * frac);
+    return (float)(before * (1.0 - frac) + now * frac);
   }
 };
 
@@ -653,7 +676,7 @@ __device__ __forceinline__ bool sequence(const Params &p, State<EXT> &s, Result 
     }
     if (T) {  // sample.rs:387-403
       if (replaying) {  // the replay reached an escape: the blocks' outcome, this window
-        tr->finish(s.n, fr, fi, p.r2, p.stripe_window, p.stripe_freq);
+        tr->end(s.n, fr, fi);
         res = tr->first;
         return true;
       }
@@ -681,7 +704,7 @@ __device__ __forceinline__ bool sequence(const Params &p, State<EXT> &s, Result 
         s.fi = EXT ? s.Zi + s.scale * s.xi : s.Zi + s.xi;
         return false;
       }
-      tr->finish(s.n, fr, fi, p.r2, p.stripe_window, p.stripe_freq);
+      tr->end(s.n, fr, fi);
     }
     return true;
   }
@@ -898,7 +921,7 @@ __device__ __forceinline__ bool settle(const Params &p, State<EXT> &s, Result &r
     if (sequence<EXT, D, L, B, T>(p, s, res, make_double2(s.Zr, s.Zi), pr, pi, fr, fi, f2, product, tr)) return true;
     if (s.n >= end) {  // the loop's end (sample.rs:237)
       if (T && s.replaying) {  // sample.rs:576-579: the replay gave up; from what was recorded
-        tr->finish(tr->first_at, tr->first_r, tr->first_i, p.r2, p.stripe_window, p.stripe_freq);
+        tr->end(tr->first_at, tr->first_r, tr->first_i);
         res = tr->first;
       } else {
         res.kind = 2;
@@ -1385,12 +1408,18 @@ __global__ void encode_jobs_kernel(const Params *__restrict__ jobs) {
 // T: the stripe variant: every lane holds a Stripe recorder and writes the Stripe column.
 template <bool T>
 struct TraceSlot {
-  __device__ __forceinline__ StripeTrace *get() { return nullptr; }
+  __device__ __forceinline__ StripeTrace *get(const Params &) { return nullptr; }
 };
 template <>
 struct TraceSlot<true> {
-  StripeTrace t;
-  __device__ __forceinline__ StripeTrace *get() { return &t; }
+#if defined(__CUDA_ARCH__)
+  __device__ __forceinline__ StripeTrace *get(const Params &p) {
+    return p.stripe_traces + ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
+  }
+#else
+  StripeTrace t;  // host builds of this header
+  StripeTrace *get(const Params &) { return &t; }
+#endif
 };
 
 // The BLA variants outside B and T store finished samples' raw state only (put's R: every
@@ -1410,7 +1439,7 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(co
   ExactProduct product;
   s.on = false;
   TraceSlot<T> trace;
-  StripeTrace *tr = trace.get();
+  StripeTrace *tr = trace.get(p);
   uint64_t t0 = p.deadline_ns ? globaltimer() : 0;
   unsigned long long n_samples = 0, iters = 0, blocks = 0, skipped = 0, fallback = 0, closed = 0;
   double shift = 0.0;
@@ -1419,8 +1448,9 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(co
   // prefix - max_iter, so that the first run counts max_iter - prefix.
   int64_t bias = 0;
   uint32_t blocks0 = 0, skipped0 = 0;  // S: the counts the run from zero started with
+  float stripe = 0.0f;  // T: of a sample that ends escaped
   auto finish = [&](uint32_t idx, const Result &r, uint64_t nblocks, uint64_t nskipped, double sh) {
-    put<B, T, L && !B && !T>(p, idx, r, T && r.kind == 0 ? tr->value : 0.0f);
+    put<B, T, L && !B && !T>(p, idx, r, T && r.kind == 0 ? stripe : 0.0f);
     uint64_t spent = (uint64_t)((int64_t)(r.kind == 2 ? p.max_iter : r.n) - bias);
     bias = 0;
     if (L) {
@@ -1503,6 +1533,18 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(co
     do {
       ended = warp_step<EXT, D, L, B, T>(p, s, res, active, done, held, thr, product, tr);
     } while (!ended);
+    if (T) {  // the windows of the samples that end escaped, one after the other by the whole warp
+#if defined(__CUDA_ARCH__)
+      __syncwarp();  // their recorders are other lanes' writes
+#endif
+      unsigned todo = __ballot_sync(FULL, ((ended >> lane) & 1u) && res.kind == 0);
+      while (todo) {
+        const unsigned l = (unsigned)__ffs((int)todo) - 1u;
+        todo &= todo - 1u;
+        const float v = (tr + ((int)l - (int)lane))->average(lane, p.r2, p.stripe_window, p.stripe_freq);
+        if (l == lane) stripe = v;
+      }
+    }
     if ((ended >> lane) & 1u) {
       done = false;
       if (S && bias > 0 && res.kind == 2) {
