@@ -36,6 +36,7 @@ struct BlaDev {
   uint32_t levels = 0;
   uint32_t off[fdk::MAX_LEVELS] = {};
   uint32_t count[fdk::MAX_LEVELS] = {};
+  bool ordered = false;  // no block's radius exceeds its first half's
   double eps = 0, dc_max = 0;
   int64_t dc_exp = 0;
 };
@@ -283,6 +284,27 @@ __global__ void pack_bla(const double *__restrict__ b7, uint64_t total, double *
     coef[2 * k + 1] = make_double2(w[2], w[3]);
     ab[k] = make_double2(w[5], w[6]);
   }
+}
+
+// bad |= 4 where a block's squared radius exceeds that of its first half (the block of half
+// its length at the same start), which no merged table has.
+struct LevelTable {
+  uint32_t levels, off[fdk::MAX_LEVELS], count[fdk::MAX_LEVELS];
+};
+
+__global__ void check_order(const double *__restrict__ r2, LevelTable t, unsigned *bad) {
+  for (uint32_t i = 1; i < t.levels; ++i)
+    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < t.count[i];
+         k += (uint64_t)gridDim.x * blockDim.x)
+      if (!(r2[t.off[i] + k] <= r2[t.off[i - 1] + 2 * k])) atomicOr(bad, 4u);
+}
+
+LevelTable level_table(const BlaDev &d) {
+  LevelTable t;
+  t.levels = d.levels;
+  std::memcpy(t.off, d.off, sizeof t.off);
+  std::memcpy(t.count, d.count, sizeof t.count);
+  return t;
 }
 
 // The fused stream: point m with the squared radii of the level-0 and level-1 blocks
@@ -644,6 +666,7 @@ fdc_status prepare(fdc_ctx *ctx, const OrbitDev &o, const fdc_job &j, fdk::Param
     p.bla_coef = o.bla.coef;
     p.bla_ab = o.bla.ab;
     p.bla_levels = o.bla.levels;
+    p.bla_ordered = o.bla.ordered ? 1u : 0u;
     std::memcpy(p.bla_off, o.bla.off, sizeof p.bla_off);
     std::memcpy(p.bla_count, o.bla.count, sizeof p.bla_count);
   }
@@ -840,12 +863,15 @@ fdc_status fdc_upload_bla(fdc_ctx *ctx, int32_t orbit, const double *blocks7, co
   if (e == cudaSuccess && total) e = upload(ctx, raw, blocks7, 56 * total);
   if (e == cudaSuccess && total) {
     pack_bla<<<grid_for(total), 256, 0, ctx->stream>>>(raw, total, d.r2, d.coef, d.ab, bad);
+    check_order<<<grid_for(d.levels > 1 ? d.count[1] : 1), 256, 0, ctx->stream>>>(d.r2, level_table(d), bad);
     e = cudaGetLastError();
   }
   pool_put(ctx, raw, 56 * total);
   unsigned flags = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&flags, bad, sizeof flags, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  d.ordered = !(flags & 4);
+  flags &= 3;
   if (e != cudaSuccess || flags) {
     free_bla(ctx, d);
     if (e != cudaSuccess) return fail(ctx, FDC_DEVICE_ERROR, std::string("BLA upload: ") + cudaGetErrorString(e));
@@ -938,6 +964,7 @@ fdc_status fdc_build_bla(fdc_ctx *ctx, int32_t orbit, double eps, double dc_max,
   e = cudaMemsetAsync(bad, 0, sizeof(unsigned), ctx->stream);
   if (e == cudaSuccess && total) {
     pack_bla<<<grid_for(total), 256, 0, ctx->stream>>>(raw, total, d.r2, d.coef, d.ab, bad);
+    check_order<<<grid_for(d.levels > 1 ? d.count[1] : 1), 256, 0, ctx->stream>>>(d.r2, level_table(d), bad);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess && export7 && total) e = download(ctx, export7, raw, 56 * total);
@@ -945,6 +972,8 @@ fdc_status fdc_build_bla(fdc_ctx *ctx, int32_t orbit, double eps, double dc_max,
   if (e == cudaSuccess) e = cudaMemcpyAsync(&badf, bad, sizeof badf, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   pool_put(ctx, buf, flag_bytes + 56 * room);
+  d.ordered = !(badf & 4);
+  badf &= 3;
   if (e != cudaSuccess || badf) {
     free_bla(ctx, d);
     if (e != cudaSuccess) return fail(ctx, FDC_DEVICE_ERROR, std::string("BLA build: ") + cudaGetErrorString(e));

@@ -55,6 +55,7 @@ struct Params {
   const double2 *__restrict__ bla_coef;
   const double2 *__restrict__ bla_ab;
   uint32_t bla_levels;
+  uint32_t bla_ordered;  // no block's radius exceeds that of its first half: levels pass as a prefix
   uint32_t bla_off[MAX_LEVELS];
   uint32_t bla_count[MAX_LEVELS];
   // frame
@@ -343,38 +344,57 @@ __device__ __forceinline__ bool block_starts(const State<EXT> &s) {
 // The rest of Bla::find once a block starts at m: the level of the longest valid block, with
 // its index in that level in `at`. Levels 1 .. top - 1 can start at m and fit: k = m - 1 is a
 // multiple of their 2^(i+1) steps, which neither the budget nor the table's last - 1 steps
-// cut short. Their radii are loaded four levels at a time before the comparisons that
-// would stop at them (the median block of the 1e-100 nucleus view is 2^7 steps long); the
-// block is the last level of the passing run (the same as testing them in order).
-template <bool EXT>
+// cut short. The reference tests them in order and stops at the first that fails. A merged
+// block's radius is at most its first half's (bla.rs:99-117; checked for every table when it
+// is uploaded or built), so the levels that pass are the first ones, and a search finds how
+// many with 6 radii in two rounds of loads instead of 8 and more: every third level, then the
+// two between (kernel ms: 2880x1620 jittered 1e-300 51.7 -> 48.7, 1920x1080 1e-100 20.0 -> 19.5,
+// tiles batch 16.7 -> 16.0). Blocks of the 1e-100 nucleus view are 2^7 steps long in the
+// median. WIDE: levels 1-8 in one round of loads, for the stripe variants, whose recorders
+// drive the table out of L1 (640x360 10.8 against 12.0 ms).
+template <bool EXT, bool WIDE>
 __device__ __forceinline__ int block_level(const Params &p, const State<EXT> &s, uint32_t &at) {
   const double d2 = block_d2(s);
   const uint32_t k = s.m - 1u;
   const uint32_t fit = min(s.lim - s.n, p.last - 1u - k);  // >= 2: a block starts here
   const uint32_t top = min(min((uint32_t)__ffs((int)k) - 1u, p.bla_levels), 31u - (uint32_t)__clz((int)fit));
+  const auto valid = [&](uint32_t i) {
+    return i < top && d2 < __ldg(p.bla_r2 + (p.bla_off[i] + (k >> (i + 1))));
+  };
   uint32_t lv = 0;
-  bool run = true;
-  constexpr uint32_t PRE = 8, MORE = 4;
-  double r[PRE];
+  if (WIDE) {
+    double r[8];
+    bool run = true;
 #pragma unroll
-  for (uint32_t q = 0; q < PRE; ++q)
-    r[q] = 1 + q < top ? __ldg(p.bla_r2 + (p.bla_off[1 + q] + (k >> (q + 2)))) : -1.0;
+    for (uint32_t q = 0; q < 8; ++q)
+      r[q] = q + 1 < top ? __ldg(p.bla_r2 + (p.bla_off[q + 1] + (k >> (q + 2)))) : -1.0;
 #pragma unroll
-  for (uint32_t q = 0; q < PRE; ++q) {
-    run = run & (d2 < r[q]);
-    lv += run;
-  }
-  if (run) {
-    for (uint32_t i = 1 + PRE; i < top && run; i += MORE) {
+    for (uint32_t q = 0; q < 8; ++q) {
+      run = run & (d2 < r[q]);
+      lv += run;
+    }
+    for (uint32_t i = 9; i < top && run; i += 4) {
 #pragma unroll
-      for (uint32_t q = 0; q < MORE; ++q)
+      for (uint32_t q = 0; q < 4; ++q)
         r[q] = i + q < top ? __ldg(p.bla_r2 + (p.bla_off[i + q] + (k >> (i + q + 1)))) : -1.0;
 #pragma unroll
-      for (uint32_t q = 0; q < MORE; ++q) {
+      for (uint32_t q = 0; q < 4; ++q) {
         run = run & (d2 < r[q]);
         lv += run;
       }
     }
+  } else if (p.bla_ordered) {
+    double r[4];
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q)
+      r[q] = 3 * q + 3 < top ? __ldg(p.bla_r2 + (p.bla_off[3 * q + 3] + (k >> (3 * q + 4)))) : -1.0;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) lv += d2 < r[q] ? 3u : 0u;
+    const bool one = valid(lv + 1), two = valid(lv + 2);
+    lv += (uint32_t)one + (uint32_t)two;
+    while (lv >= 14 && valid(lv + 1)) ++lv;
+  } else {
+    while (valid(lv + 1)) ++lv;
   }
   at = k >> (lv + 1);
   return (int)lv;
@@ -1116,7 +1136,7 @@ __device__ __forceinline__ unsigned warp_step(const Params &p, State<EXT> &s, Re
     ended = __ballot_sync(FULL, done);
     if (wait && !done) {
       uint32_t at;
-      const int lv = block_level(p, s, at);
+      const int lv = block_level<EXT, T>(p, s, at);
       if (T)  // sample.rs:267-281: the block start, for a later replay
         tr->snap(StripeSnap{s.m, s.n, s.xr, s.xi, s.delta_exp, s.scale, s.dc_r, s.dc_i, 0}, s.n + (2u << lv));
       apply_block<EXT, D>(p, s, lv, at, product);
