@@ -100,10 +100,24 @@ struct StateF {
   MulF mu, ct;
   bool ct_started;
   uint32_t n, chk, sn, hold, m, idx, blocks, skipped;
-  uint32_t lim;  // relimit_f32()
+  uint32_t lim;   // relimit_f32()
+  uint32_t stop;  // the next iterate at which something may come due, <= lim
+  float near;     // the near-return bound of the save point, infinite while a save is pending
   int nucleus;
+  bool on;  // the next operation is a BLA block (set by post_f32)
   bool pending, predicted;
 };
+
+__device__ __forceinline__ void save_f32(StateF &s, float r, float i) {
+  s.sr = r;
+  s.si = i;
+  s.near = 1e-3f * (fabsf(r) + fabsf(i));
+}
+
+__device__ __forceinline__ void await_save_f32(StateF &s) {
+  s.pending = true;
+  s.near = __int_as_float(0x7f800000);
+}
 
 // delta = (re, im) 2^k (f64 mantissas, any k) into the f32 form, the exponent kept at or
 // above oe - 64 so that dc 2^-e stays representable.
@@ -182,6 +196,7 @@ __device__ __forceinline__ void relimit_f32(const Params &p, StateF &s) {
   uint64_t b = p.max_iter < cap ? p.max_iter : cap;
   if (s.nucleus >= 0 && (uint64_t)s.nucleus + 1 < b) b = (uint64_t)s.nucleus + 1;
   s.lim = (uint32_t)b;
+  s.stop = below_f64(p) ? min(s.lim, s.chk) : s.lim;
 }
 
 // Whether Bla::find (on the FP64 |delta|^2 of the iteration's start, s.d2) finds a block.
@@ -284,7 +299,7 @@ __device__ __forceinline__ void plain_update_f32(StateF &s) {
     double t = 2.0 * (s.fr * s.dr - s.fi * s.di) + s.inverse;
     s.di = 2.0 * (s.fr * s.di + s.fi * s.dr);
     s.dr = t;
-    if (fmax(fabs(s.dr), fabs(s.di)) > HI) {
+    if ((fabs(s.dr) > HI) | (fabs(s.di) > HI)) {
       s.dr = s.dr * LO;
       s.di = s.di * LO;
       s.dexp += 32;
@@ -339,27 +354,11 @@ static __device__ __noinline__ Newton newton(MulF mu, float gr, float gi, float 
   return n;
 }
 
-// After the update: next entry, FP64 bailout and rebase test, FP32 periodicity. nz/nr
-// hold the entry m + 1 prefetched at the iteration's start (after a plain step); after a
-// block (took) the entry at the new m is loaded here.
-template <bool D, bool L>
-__device__ __forceinline__ bool post_f32(const Params &p, const Entry32 *__restrict__ orbit, StateF &s,
-                                         Result &res, bool took, double2 nz, double2 nr) {
-  double2 Z = nz;
-  if (took) {
-    const double2 *e3 = reinterpret_cast<const double2 *>(orbit + s.m);
-    Z = __ldg(e3);
-    nr = __ldg(e3 + 1);
-  }
-  s.Zr = Z.x;
-  s.Zi = Z.y;
-  s.zr32 = __int_as_float((int)(__double_as_longlong(nr.x) & 0xffffffffll));
-  s.zi32 = __int_as_float((int)(__double_as_longlong(nr.x) >> 32));
-  s.r2a = nr.y;
-  // FP64: the physical delta, z, the bailout and the rebase test
-  const double pr = phys(s.wr, s.e, s.s64), pi = phys(s.wi, s.e, s.s64);
-  const double fr = Z.x + pr, fi = Z.y + pi;
-  const double f2 = fr * fr + fi * fi;
+// The full sequence of an iteration in which something may have happened (sample.rs:381-575
+// by the extended tier's rebase rule and the ordinary tier's periodicity): z = (fr, fi) with
+// |z|^2 = f2, the physical delta's square delta2. Returns true when the sample has an outcome.
+__device__ __forceinline__ bool sequence_f32(const Params &p, StateF &s, Result &res, double fr, double fi, double f2,
+                                             double delta2, bool reb) {
   if (f2 > p.r2) {
     res.kind = 0;
     res.n = s.n;
@@ -379,12 +378,11 @@ __device__ __forceinline__ bool post_f32(const Params &p, const Entry32 *__restr
     s.nucleus = -1;
     relimit_f32(p, s);
   }
-  const double delta2 = pr * pr + pi * pi;
-  if (f2 <= delta2 || s.m == p.last) {  // rebase onto Z_0 (extended-tier rule)
+  if (reb) {  // rebase onto Z_0 (extended-tier rule)
     if (f2 > SQUARE_OK) {
       set_delta(s, fr, fi, 0);
     } else {  // z below f64's reach: Z + delta with wide exponents (sample.rs:421-429)
-      const Cx3 t = add3(Cx3{Z.x, Z.y, 0}, Cx3{(double)s.wr, (double)s.wi, s.e});
+      const Cx3 t = add3(Cx3{s.Zr, s.Zi, 0}, Cx3{(double)s.wr, (double)s.wi, s.e});
       set_delta(s, t.re, t.im, t.e);
     }
     s.m = 0;
@@ -411,8 +409,7 @@ __device__ __forceinline__ bool post_f32(const Params &p, const Entry32 *__restr
       // blocks run each sample to the orbit's last point, whose rebase onto z = Z_last
       // (delta below f64) would put every sample on the reference orbit.
       if (s.n >= s.chk) {
-        s.sr = (float)fr;
-        s.si = (float)fi;
+        save_f32(s, (float)fr, (float)fi);
         s.sn = s.n;
         s.chk = s.chk >= 0x80000000u ? 0xffffffffu : s.chk * 2;
         relimit_f32(p, s);
@@ -421,11 +418,11 @@ __device__ __forceinline__ bool post_f32(const Params &p, const Entry32 *__restr
       if (s.n >= s.sn + s.hold) {
         s.hold = 0;
         s.predicted = false;
-        s.pending = true;
+        await_save_f32(s);
         relimit_f32(p, s);
       }
     } else if (s.n >= s.chk) {
-      s.pending = true;
+      await_save_f32(s);
       relimit_f32(p, s);
     }
     return false;
@@ -450,8 +447,7 @@ __device__ __forceinline__ bool post_f32(const Params &p, const Entry32 *__restr
       s.predicted = false;
     }
     s.hold = period;
-    s.sr = gr;
-    s.si = gi;
+    save_f32(s, gr, gi);
     s.sn = s.n;
     s.pending = false;
     s.mu.reset();
@@ -462,13 +458,12 @@ __device__ __forceinline__ bool post_f32(const Params &p, const Entry32 *__restr
     if (s.n < s.sn + s.hold) return false;
     s.hold = 0;
     s.predicted = false;
-    s.pending = true;
+    await_save_f32(s);
   }
   if (s.pending || s.n >= s.chk) {
     uint32_t np = (uint32_t)next_pow2((uint64_t)s.n + 1);
     s.chk = s.chk > np ? s.chk : np;
-    s.sr = gr;
-    s.si = gi;
+    save_f32(s, gr, gi);
     s.sn = s.n;
     s.pending = false;
   }
@@ -476,57 +471,82 @@ __device__ __forceinline__ bool post_f32(const Params &p, const Entry32 *__restr
   return false;
 }
 
-// A lane's BLA block found but not yet applied.
-struct Waiting {
-  bool on;
-  int lv;
-  uint32_t at;
-};
-
-// One iteration of the precision form for the active lanes of a warp, with the block
-// deferral of warp_step.
+// After the update: the next entry, FP64 bailout and rebase test, FP32 periodicity, and the
+// choice of the next operation. nz/nr hold the entry m + 1 prefetched at the iteration's
+// start (after a plain step); after a block (took) the entry at the new m is loaded here.
+// As the plain form's post, a common iteration carries z and one test, true without cause
+// at times and never false with one, sends every other to the full sequence: issue slots and
+// instruction fetch bound this kernel, and a region for each condition took most of them.
 template <bool D, bool L>
-__device__ __forceinline__ bool warp_step_f32(const Params &p, const Entry32 *__restrict__ orbit, StateF &s,
-                                              Result &res, bool active, Waiting &w, uint32_t defer) {
-  bool upd = false, took = false, done = false;
-  double2 nz = make_double2(0.0, 0.0), nr = make_double2(0.0, -1.0);
-  if (active && !w.on) {
+__device__ __forceinline__ bool post_f32(const Params &p, const Entry32 *__restrict__ orbit, StateF &s,
+                                         Result &res, bool took, double2 nz, double2 nr) {
+  double2 Z = nz;
+  if (took) {
+    const double2 *e3 = reinterpret_cast<const double2 *>(orbit + s.m);
+    Z = __ldg(e3);
+    nr = __ldg(e3 + 1);
+  }
+  s.Zr = Z.x;
+  s.Zi = Z.y;
+  s.zr32 = __int_as_float((int)(__double_as_longlong(nr.x) & 0xffffffffll));
+  s.zi32 = __int_as_float((int)(__double_as_longlong(nr.x) >> 32));
+  s.r2a = nr.y;
+  // FP64: the physical delta, z, the bailout and the rebase test
+  const double pr = phys(s.wr, s.e, s.s64), pi = phys(s.wi, s.e, s.s64);
+  const double fr = Z.x + pr, fi = Z.y + pi;
+  const double f2 = fr * fr + fi * fi;
+  const double delta2 = pr * pr + pi * pi;
+  const uint32_t f2_hi = (uint32_t)__double2hiint(f2);
+  const bool reb = f2 <= delta2 || s.m == p.last;
+  bool rare = (f2_hi >= (uint32_t)__double2hiint(p.r2)) | reb | (s.n >= s.stop);
+  // a near return counts where |delta|^2 > 1e-24 |z|^2: for no high words 80 binades apart
+  const float gr = (float)fr, gi = (float)fi;
+  rare |= (fabsf(gr - s.sr) + fabsf(gi - s.si) < s.near) & ((uint32_t)__double2hiint(delta2) + (80u << 20) > f2_hi);
+  if (__builtin_expect(rare, 0)) {
+    if (sequence_f32(p, s, res, fr, fi, f2, delta2, reb)) return true;
     if (s.n >= p.max_iter) {
       res.kind = 2;
-      done = true;
-    } else {
-      // speculative load of the next entry (m < last at the top of every iteration)
-      const double2 *e2 = reinterpret_cast<const double2 *>(orbit + s.m + 1);
-      nz = __ldg(e2);
-      nr = __ldg(e2 + 1);
-      // a lane that finds a block waits; its level is searched when the waiting lanes
-      // apply their blocks together (nothing the search reads changes while it waits)
-      if (L && block_starts_f32(s)) {
-        w.on = true;
-      } else {
-        plain_update_f32<D>(s);
-        upd = true;
-      }
+      return true;
     }
+    s.on = L && block_starts_f32(s);
+    return false;
   }
-  if (L) {
-    const unsigned FULL = 0xffffffffu;
-    const unsigned waiting = __ballot_sync(FULL, w.on);
-    const unsigned stepping = __ballot_sync(FULL, upd);
-    // the threshold is `defer` of 32 lanes, scaled to the lanes still busy (waiting or
-    // stepping): once the queue runs dry and lanes go idle, a fixed threshold would hold
-    // every waiting lane until the last plain-stepping lane finds a block
-    const uint32_t busy = (uint32_t)__popc(waiting | stepping);
-    const uint32_t thr = max(1u, (busy * defer) >> 5);
-    if (waiting && ((uint32_t)__popc(waiting) >= thr || !stepping) && w.on) {
-      w.lv = block_level_f32(p, s, w.at);
-      apply_block_f32<D>(p, s, w.lv, w.at);
-      w.on = false;
+  s.d2 = delta2;
+  s.fr = fr;
+  s.fi = fi;
+  if (L) s.on = (delta2 < s.r2a) & (s.n + 1u < s.lim);  // no block starts at Z_0
+  return false;
+}
+
+// One iteration of the precision form for the lanes of a warp that hold a sample, with
+// warp_step's deferral of blocks and outcomes.
+template <bool D, bool L>
+__device__ __forceinline__ unsigned warp_step_f32(const Params &p, const Entry32 *__restrict__ orbit, StateF &s,
+                                                  Result &res, bool active, bool &done, unsigned held, uint32_t thr) {
+  const unsigned FULL = 0xffffffffu;
+  const bool wait = s.on | done;  // neither in a lane without a sample
+  bool upd = active && !wait, took = false;
+  double2 nz = make_double2(0.0, 0.0), nr = make_double2(0.0, -1.0);
+  if (upd) {
+    // speculative load of the next entry (m < last at the top of every iteration)
+    const double2 *e2 = reinterpret_cast<const double2 *>(orbit + s.m + 1);
+    nz = __ldg(e2);
+    nr = __ldg(e2 + 1);
+    plain_update_f32<D>(s);
+  }
+  const unsigned waiting = __ballot_sync(FULL, wait);
+  unsigned ended = 0;
+  if ((uint32_t)__popc(waiting) >= (L ? thr : 1u) || waiting == held) {
+    ended = __ballot_sync(FULL, done);
+    if (L && wait && !done) {
+      uint32_t at;
+      const int lv = block_level_f32(p, s, at);
+      apply_block_f32<D>(p, s, lv, at);
       upd = took = true;
     }
   }
   if (upd) done = post_f32<D, L>(p, orbit, s, res, took, nz, nr);
-  return done;
+  return ended;
 }
 
 template <bool D, bool L>
@@ -579,7 +599,8 @@ __device__ __forceinline__ int init_f32(const Params &p, uint64_t slot, StateF &
   s.inverse = 1.0;
   s.m = 0;
   s.n = 0;
-  s.sr = s.si = 0.0f;
+  save_f32(s, 0.0f, 0.0f);
+  s.on = false;
   s.chk = 16;
   s.sn = 8;
   s.pending = false;
@@ -603,8 +624,8 @@ __global__ void __launch_bounds__(128, FDK_MIN_BLOCKS_F32) perturb_f32_kernel(Pa
   const unsigned lt = (1u << lane) - 1u;
   StateF s;
   Result res;
-  Waiting w{false, -1, 0};
-  bool active = false, exhausted = false;
+  bool active = false, done = false, exhausted = false;
+  s.on = false;
   uint64_t t0 = p.deadline_ns ? globaltimer() : 0;
   unsigned long long n_samples = 0, iters = 0, blocks = 0, skipped = 0, fallback = 0, closed = 0;
   // the BLA variants store a finished sample's raw state; encode_kernel computes its nu, de
@@ -648,16 +669,27 @@ __global__ void __launch_bounds__(128, FDK_MIN_BLOCKS_F32) perturb_f32_kernel(Pa
         uint64_t slot = base + __popc(need & lt);
         if (slot < p.total) {
           int got = init_f32<D, L>(p, slot, s, res);
-          if (got == 1) active = true;
-          else if (got == 2) finish(s.idx, res, 0, 0);
+          active = got == 1 && s.n < p.max_iter;
+          if (got != 0 && !active) {  // settled, or no iteration to run
+            if (got == 1) res.kind = 2;
+            finish(s.idx, res, 0, 0);
+          }
         }
       }
       need = __ballot_sync(FULL, !active);
     }
-    if (!__any_sync(FULL, active)) break;
-    if (warp_step_f32<D, L>(p, orbit, s, res, active, w, p.defer)) {
+    const unsigned held = __ballot_sync(FULL, active);
+    if (!held) break;
+    const uint32_t thr = threshold(held, p.defer);
+    unsigned ended = 0;
+    do {
+      ended = warp_step_f32<D, L>(p, orbit, s, res, active, done, held, thr);
+    } while (!ended);
+    if ((ended >> lane) & 1u) {
+      done = false;
       finish(s.idx, res, s.blocks, s.skipped);
       active = false;
+      s.on = false;
     }
   }
   for (int o = 16; o > 0; o >>= 1) {
@@ -695,8 +727,8 @@ __global__ void __launch_bounds__(128, FDK_MIN_BLOCKS_F32)
   const unsigned lt = (1u << lane) - 1u;
   StateF s;
   Result res;
-  Waiting w{false, -1, 0};
-  bool active = false, exhausted = false;
+  bool active = false, done = false, exhausted = false;
+  s.on = false;
   uint32_t job = 0, counted = 0xffffffffu;
   LaneCounters lc;
   lc.clear();
@@ -736,17 +768,28 @@ __global__ void __launch_bounds__(128, FDK_MIN_BLOCKS_F32)
           job = job_of(starts, njobs, slot);
           const Params &p = jobs[job];
           int got = init_f32<D, L>(p, slot - __ldg(starts + job), s, res);
-          if (got == 1) active = true;
-          else if (got == 2) finish(p, s.idx, res, 0, 0);
+          active = got == 1 && s.n < p.max_iter;
+          if (got != 0 && !active) {  // settled, or no iteration to run
+            if (got == 1) res.kind = 2;
+            finish(p, s.idx, res, 0, 0);
+          }
         }
       }
       need = __ballot_sync(FULL, !active);
     }
-    if (!__any_sync(FULL, active)) break;
+    const unsigned held = __ballot_sync(FULL, active);
+    if (!held) break;
+    const uint32_t thr = threshold(held, defer);
     const Params &p = jobs[job];
-    if (warp_step_f32<D, L>(p, (const Entry32 *)p.orbit32, s, res, active, w, defer)) {
+    unsigned ended = 0;
+    do {
+      ended = warp_step_f32<D, L>(p, (const Entry32 *)p.orbit32, s, res, active, done, held, thr);
+    } while (!ended);
+    if ((ended >> lane) & 1u) {
+      done = false;
       finish(p, s.idx, res, s.blocks, s.skipped);
       active = false;
+      s.on = false;
     }
   }
   if (counted != 0xffffffffu) lc.flush(per_job + counted);
