@@ -159,6 +159,32 @@ __device__ __forceinline__ void set_delta(StateF &s, double re, double im, int64
   s.dci = d.dci;
 }
 
+// delta = (r1, i1) 2^e1 + (r2, i2) 2^e2 as set_delta stores add3's sum, without the wide
+// exponents: scaling by a power of two is exact, so the sum may be taken at e1 wherever its
+// parts are within 2^400 of each other and of moderate size (a term too small for binary64 at
+// either scale then vanishes in both; a part is zero only with a zero or cancelled term).
+// False, with nothing changed, for any other sum.
+__device__ __forceinline__ bool quick_delta(StateF &s, double r1, double i1, int e1, double r2, double i2, int e2) {
+  constexpr uint32_t ONE = 1023u << 20;
+  const double f = exp2i(e2 - e1);
+  const double re = r1 + r2 * f, im = i1 + i2 * f;
+  const uint32_t a = magnitude_hi(re), b = magnitude_hi(im), top = max(a, b), low = min(a, b);
+  if (!((low >= ONE - (600u << 20)) & (top < ONE + (600u << 20)) & (top - low <= (400u << 20)) & (e2 - e1 < 600)))
+    return false;
+  const int e = max(e1 + (int)(top >> 20) - 1023, s.oe - 64);
+  if (e1 - e < -1000) return false;
+  const double h = pow2(e1 - e);
+  s.wr = (float)(re * h);
+  s.wi = (float)(im * h);
+  s.e = e;
+  s.s32 = exp2f_int(e);
+  s.s64 = exp2i(e);
+  const double g = exp2i(s.oe - e);
+  s.dcr = (float)(s.ar * g);
+  s.dci = (float)(s.ai * g);
+  return true;
+}
+
 // Sum of two wide-exponent complex terms (as sum2, sample.rs:1094-1114), with a zero
 // term passed over: sum2 scales every term by 2^(e - top), and a zero term whose
 // exponent lies more than 2046 above the other's (an orbit point that is 0 in f64 next
@@ -258,6 +284,23 @@ static __device__ __noinline__ DzF block_dz(double dr, double di, int64_t dexp, 
   return DzF{dr, di, exp2i(-dexp), dexp};
 }
 
+// The same with one normalisation where block_fits holds (perturb_f64.cuh).
+__device__ __forceinline__ bool block_dz_quick(StateF &s, double2 A, double2 B) {
+  const uint32_t bh = max(magnitude_hi(B.x), magnitude_hi(B.y)), dh = max(magnitude_hi(s.dr), magnitude_hi(s.di));
+  const double dr = A.x * s.dr - A.y * s.di + B.x * s.inverse;
+  const double di = A.x * s.di + A.y * s.dr + B.y * s.inverse;
+  const uint32_t drh = magnitude_hi(dr), dih = magnitude_hi(di), dtop = max(drh, dih);
+  if (!(block_fits(dh, dtop, min(drh, dih), bh) & (__double2hiint(s.inverse) - (int)dh <= (int)(900u << 20))))
+    return false;
+  const int k = (int)(dtop >> 20) - 1023;
+  const double f = pow2(-k);
+  s.dr = dr * f;
+  s.di = di * f;
+  s.dexp += k;
+  s.inverse = exp2i(-s.dexp);
+  return true;
+}
+
 // delta' = A delta + B dc with wide exponents, dz' = A dz + B in FP64.
 template <bool D>
 __device__ __forceinline__ void apply_block_f32(const Params &p, StateF &s, int lv, uint32_t at) {
@@ -269,7 +312,7 @@ __device__ __forceinline__ void apply_block_f32(const Params &p, StateF &s, int 
     s.ct_started = true;
   }
   if (s.hold > 0) s.mu.multiply_wide(A.x, A.y);
-  if (D) {
+  if (D && !block_dz_quick(s, A, B)) {
     DzF z = block_dz(s.dr, s.di, s.dexp, A, B);
     s.dr = z.dr;
     s.di = z.di;
@@ -279,8 +322,10 @@ __device__ __forceinline__ void apply_block_f32(const Params &p, StateF &s, int 
   const double wr = s.wr, wi = s.wi;
   Cx3 ad{A.x * wr - A.y * wi, A.x * wi + A.y * wr, s.e};
   Cx3 bd{B.x * s.ar - B.y * s.ai, B.x * s.ai + B.y * s.ar, s.oe};
-  Cx3 d = add3(ad, bd);
-  set_delta(s, d.re, d.im, d.e);
+  if (!quick_delta(s, ad.re, ad.im, s.e, bd.re, bd.im, s.oe)) {
+    Cx3 d = add3(ad, bd);
+    set_delta(s, d.re, d.im, d.e);
+  }
   s.m += len;
   s.n += len;
   s.blocks += 1;
@@ -315,15 +360,21 @@ __device__ __forceinline__ void plain_update_f32(StateF &s) {
     s.wr = nwr;
     s.wi = nwi;
     const float mag = fmaxf(fabsf(nwr), fabsf(nwi));
-    if (mag > 4294967296.0f || (mag < 2.3283064e-10f && s.e > s.oe - 64)) set_delta(s, nwr, nwi, s.e);
+    if (mag > 4294967296.0f || (mag < 2.3283064e-10f && s.e > s.oe - 64)) {
+      if (!quick_delta(s, nwr, nwi, s.e, 0.0, 0.0, s.e)) set_delta(s, nwr, nwi, s.e);
+    }
   } else {
     // exact step at a tiny Z_m: 2 Z delta + delta^2 + dc with wide exponents
     const double wr = s.wr, wi = s.wi;
     Cx3 zd{2.0 * (s.Zr * wr - s.Zi * wi), 2.0 * (s.Zr * wi + s.Zi * wr), s.e};
     Cx3 dd{wr * wr - wi * wi, 2.0 * wr * wi, 2 * (int64_t)s.e};
     Cx3 a{s.ar, s.ai, s.oe};
-    Cx3 t = add3(add3(zd, dd), a);
-    set_delta(s, t.re, t.im, t.e);
+    // from Z_0 = 0, one step in 8 with the rebases, delta^2 + dc
+    const bool zero = s.Zr == 0.0 && s.Zi == 0.0 && (dd.re != 0.0 || dd.im != 0.0);
+    if (!zero || !quick_delta(s, dd.re, dd.im, 2 * s.e, s.ar, s.ai, s.oe)) {
+      Cx3 t = add3(add3(zd, dd), a);
+      set_delta(s, t.re, t.im, t.e);
+    }
   }
   s.m += 1;
   s.n += 1;
@@ -380,7 +431,7 @@ __device__ __forceinline__ bool sequence_f32(const Params &p, StateF &s, Result 
   }
   if (reb) {  // rebase onto Z_0 (extended-tier rule)
     if (f2 > SQUARE_OK) {
-      set_delta(s, fr, fi, 0);
+      if (!quick_delta(s, fr, fi, 0, 0.0, 0.0, 0)) set_delta(s, fr, fi, 0);
     } else {  // z below f64's reach: Z + delta with wide exponents (sample.rs:421-429)
       const Cx3 t = add3(Cx3{s.Zr, s.Zi, 0}, Cx3{(double)s.wr, (double)s.wi, s.e});
       set_delta(s, t.re, t.im, t.e);
