@@ -113,10 +113,11 @@ struct fdc_ctx {
 // extended tier's blocks carry renormalisations and gather more lanes. Kernel ms over 4, 6,
 // 8, 10, 12, 16: 1920x1080 at a 1e-100 nucleus, extended tier 27.2 25.6 24.3 23.6 23.3 24.1;
 // 1280x720 on the Fixed tier 11.7 12.1 12.5 12.6 13.1 14.2.
-// The precision form's own defaults are 12 and 8.
+// The precision form over 2, 3, 4, 6, 8, 12: 960x540 at 1e-100, extended tier 9.52 9.59 9.77 9.95 10.06
+// 10.48; at 1e-70 on the Fixed tier 6.04 5.93 5.90 5.74 5.73 5.76.
 static uint32_t defer_for(const fdc_ctx *ctx, bool ext, bool f32) {
   if (ctx->tune.defer > 0) return ctx->tune.defer;
-  return ext ? 12u : (f32 ? 8u : 4u);
+  return f32 ? (ext ? 3u : 8u) : (ext ? 12u : 4u);
 }
 
 // The tiles of a window, nearest to its centre first (squared distance of the tile's
@@ -1172,6 +1173,17 @@ fdc_status render_impl(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, const fdc
   p.timed_out = &ctx->scratch->timed_out;
   CK(cudaMemsetAsync(ctx->scratch, 0, sizeof(Scratch), ctx->stream));
 
+  const uint64_t resident = ext && !(j.flags & FDC_F32) ? fdk::Occupancy<true>::blocks : fdk::Occupancy<false>::blocks;
+  // A launch of few samples spreads them over 12 warps an SM instead of filling the first
+  // warps: a warp of 32 lanes that diverge runs every lane's branches and waits for every
+  // lane's table loads (kernel ms at full warps / 4, 8, 12, 16 warps an SM: 64x36 shallow
+  // 0.418 / 0.343 0.333 0.329 0.351, 161x91 with blocks 1.12 / 1.09 0.95 0.85 0.94).
+  // Over the last three waves of the grid a warp reserves no slots ahead (401x227 without a
+  // table 1.15 -> 0.86 ms, 480x270 2.72 -> 2.49; an eighth of the queue where that is more).
+  const uint64_t spread = (uint64_t)ctx->sm_count * 12, lanes = (p.total + spread - 1) / spread;
+  p.idle_lanes = lanes < 32 ? (uint32_t)(32 - lanes) : 0;
+  p.tail = (uint32_t)std::max<uint64_t>(p.total / 8, 3ull * ctx->sm_count * resident * 128);
+
   uint32_t launches = 1;
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   if (j.flags & FDC_F32) {
@@ -1191,15 +1203,6 @@ fdc_status render_impl(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, const fdc
       ctx->blocks_per_sm[variant] = b > 0 ? b : 1;
     }
     dim3 grid(grid_blocks(ctx, ctx->blocks_per_sm[variant])), block(128);
-    // A launch of few samples spreads them over 12 warps an SM instead of filling the first
-    // warps: a warp of 32 lanes that diverge runs every lane's branches and waits for every
-    // lane's table loads (kernel ms at full warps / 4, 8, 12, 16 warps an SM: 64x36 shallow
-    // 0.418 / 0.343 0.333 0.329 0.351, 161x91 with blocks 1.12 / 1.09 0.95 0.85 0.94).
-    // Over the last three waves of the grid a warp reserves no slots ahead (401x227 without a
-    // table 1.15 -> 0.86 ms, 480x270 2.72 -> 2.49; an eighth of the queue where that is more).
-    const uint64_t spread = (uint64_t)ctx->sm_count * 12, lanes = (p.total + spread - 1) / spread;
-    p.idle_lanes = lanes < 32 ? (uint32_t)(32 - lanes) : 0;
-    p.tail = (uint32_t)std::max<uint64_t>(p.total / 8, 3ull * grid.x * block.x);
     const size_t trace_bytes = stripe ? sizeof(fdk::StripeTrace) * grid.x * block.x : 0;
     if (stripe) {
       p.stripe_traces = (fdk::StripeTrace *)pool_get(ctx, trace_bytes);

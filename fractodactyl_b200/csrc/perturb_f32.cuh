@@ -695,8 +695,11 @@ __global__ void __launch_bounds__(128, FDK_MIN_BLOCKS_F32) perturb_f32_kernel(Pa
     iters += spent;
     n_samples += 1;
   };
+  const unsigned taking = FULL >> p.idle_lanes;
+  Reservation slots;
+  slots.tail = p.idle_lanes != 0;
   for (;;) {
-    unsigned need = __ballot_sync(FULL, !active);
+    unsigned need = __ballot_sync(FULL, !active) & taking;
     while (need && !exhausted) {
       if (p.deadline_ns) {
         uint64_t now = 0;
@@ -709,16 +712,15 @@ __global__ void __launch_bounds__(128, FDK_MIN_BLOCKS_F32) perturb_f32_kernel(Pa
         }
       }
       unsigned long long base = 0;
-      int leader = __ffs((int)need) - 1;
-      if ((int)lane == leader) base = atomicAdd(p.queue, (unsigned long long)__popc(need));
-      base = __shfl_sync(FULL, base, leader);
-      if (base >= p.total) {
+      unsigned take = 0;
+      if (!slots.take(p.queue, p.total, p.tail, need, lane, base, take)) {
         exhausted = true;
         break;
       }
-      if (!active) {
-        uint64_t slot = base + __popc(need & lt);
-        if (slot < p.total) {
+      if (!active && ((need >> lane) & 1u)) {
+        const unsigned rank = __popc(need & lt);
+        const uint64_t slot = base + rank;
+        if (rank < take) {
           int got = init_f32<D, L>(p, slot, s, res);
           active = got == 1 && s.n < p.max_iter;
           if (got != 0 && !active) {  // settled, or no iteration to run
@@ -727,7 +729,7 @@ __global__ void __launch_bounds__(128, FDK_MIN_BLOCKS_F32) perturb_f32_kernel(Pa
           }
         }
       }
-      need = __ballot_sync(FULL, !active);
+      need = __ballot_sync(FULL, !active) & taking;
     }
     const unsigned held = __ballot_sync(FULL, active);
     if (!held) break;
@@ -781,6 +783,8 @@ __global__ void __launch_bounds__(128, FDK_MIN_BLOCKS_F32)
   bool active = false, done = false, exhausted = false;
   s.on = false;
   uint32_t job = 0, counted = 0xffffffffu;
+  Reservation slots;
+  const unsigned long long waves = 3ull * gridDim.x * blockDim.x, last = waves > total / 8 ? waves : total / 8;
   LaneCounters lc;
   lc.clear();
   // as the plain batch kernel: the BLA variants store raw state for encode_jobs_kernel
@@ -806,16 +810,15 @@ __global__ void __launch_bounds__(128, FDK_MIN_BLOCKS_F32)
     unsigned need = __ballot_sync(FULL, !active);
     while (need && !exhausted) {
       unsigned long long base = 0;
-      int leader = __ffs((int)need) - 1;
-      if ((int)lane == leader) base = atomicAdd(queue, (unsigned long long)__popc(need));
-      base = __shfl_sync(FULL, base, leader);
-      if (base >= total) {
+      unsigned take = 0;
+      if (!slots.take(queue, total, last, need, lane, base, take)) {
         exhausted = true;
         break;
       }
       if (!active) {
-        unsigned long long slot = base + __popc(need & lt);
-        if (slot < total) {
+        const unsigned rank = __popc(need & lt);
+        const unsigned long long slot = base + rank;
+        if (rank < take) {
           job = job_of(starts, njobs, slot);
           const Params &p = jobs[job];
           int got = init_f32<D, L>(p, slot - __ldg(starts + job), s, res);
