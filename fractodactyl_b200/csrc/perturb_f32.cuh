@@ -7,7 +7,8 @@
 //   4. the derivative dz/dc for distance estimates (sample.rs:352-360).
 // Periodicity, the nucleus contraction and Newton's cycle prediction run in FP32.
 // Steps from an orbit point whose FP32 copy is not exact enough (|Z| < 2^-60: Z_0 and a
-// nucleus's returns) and BLA block applications use wide-exponent FP64 arithmetic.
+// nucleus's returns) and BLA block applications use FP64 arithmetic, with wide exponents where
+// binary64's range does not hold their terms (quick_delta).
 // Compiled with fused multiply-adds (this form is not bit-exact by design).
 #pragma once
 #include <cstdint>

@@ -1,9 +1,10 @@
 // The plain (FP64) perturbation kernel: one lane per sample, persistent warps that
 // refill finished lanes from an atomic tile queue. The per-sample state machine is
 // iterate() of crates/fd-kernel/src/sample.rs:170-581 (Binary64 and Binary64Exponent,
-// number.rs:92-124) with the reference's operation order: one loop iteration is
-// find_block, then apply_block or plain_update, then post; warp_step runs it for a
-// warp (with BLA deferral), step for one lane. Compile with -fmad=false.
+// number.rs:92-124) with the reference's operation order: one loop iteration is apply_block
+// or plain_update, then post, which tests for rare events once (settle handles them) and
+// chooses the next operation; warp_step runs it for a warp (with BLA deferral), step for
+// one lane. Compile with -fmad=false.
 #pragma once
 #include <cstdint>
 
@@ -40,8 +41,8 @@ struct StripeTrace;
 struct Params {
   const double2 *__restrict__ orbit;  // Z_0..Z_last, interleaved re/im
   // With BLA: Z_m fused with the squared radii of the level-1 and level-2 blocks (j = 1, 2)
-  // starting at m, or -1 where none starts there: 32-byte entries (zr, zi, r2a, r2b), so the
-  // first two levels of Bla::find come with the orbit point each step loads anyway.
+  // starting at m, or -1 where none starts there: 32-byte entries (zr, zi, r2a, r2b), one load
+  // each, so that whether a block starts comes with the orbit point each step loads anyway.
   const double2 *__restrict__ fused;
   const void *orbit32;  // precision-form entries (perturb_f32.cuh), per job in batches
   uint32_t last;
@@ -936,10 +937,12 @@ __device__ __forceinline__ bool sequence(const Params &p, State<EXT> &s, Result 
   return false;
 }
 
-// The end of an iteration in which something may have happened: the derivative's rescaling
-// (dbig), an event of the full sequence, a rebase (reb), a rescaling of the delta, a due
-// periodicity check (limit), a near return, a block radius below binary64's squares, or a
-// contraction product leaving its range. Each part tests its own condition exactly.
+// The end of an iteration in which something may have happened: the derivative's rescaling,
+// an event of the full sequence (wild: |z|^2 out of the quiet range), a rebase (reb), a
+// rescaling of the delta, a due periodicity check, a near return, a block radius below
+// binary64's squares, or a contraction product leaving its range. Each part tests its own
+// condition exactly. Rebases and checks keep short forms of their own here: run through the
+// full sequence they took the 1920x1080 1e-100 frame from 20.4 to 22.7 ms.
 template <bool EXT, bool D, bool L, bool B, bool T>
 __device__ __forceinline__ bool settle(const Params &p, State<EXT> &s, Result &res, double pr, double pi,
                                        double fr, double fi, double f2, double delta2, bool reb, bool wild,
