@@ -16,8 +16,9 @@ constexpr int MAX_LEVELS = 40;
 
 // Resident 128-thread blocks per SM each kernel variant is compiled for (caps registers
 // at 65536 / (128 * blocks)): floatexp-tier variants (EXT) and ordinary-tier variants;
-// chosen by measurement (5 floatexp blocks at 96 registers: the 1920x1080 frame at a 1e-100
-// nucleus, 10^6 iterations, 37.95 -> 37.53 ms).
+// chosen by measurement. Kernel ms at 4 / 5 / 6 floatexp blocks: 1920x1080 at a 1e-100 nucleus
+// 20.3 / 19.5 / 20.0, 2880x1620 jittered at 1e-300 50.8 / 48.7 / 49.5; at 3 / 4 / 5 ordinary
+// ones: 1280x720 with blocks 9.7 / 10.1 / 11.0, 480x270 without 2.97 / 2.53 / 2.59.
 #ifndef FDK_MIN_BLOCKS_EXT
 #define FDK_MIN_BLOCKS_EXT 5
 #endif
