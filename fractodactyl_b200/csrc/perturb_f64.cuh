@@ -1491,7 +1491,8 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(Pa
   // on a first run from the series (> 0); after an unresolved first run retried from zero,
   // prefix - max_iter, so that the first run counts max_iter - prefix.
   int64_t bias = 0;
-  uint32_t blocks0 = 0, skipped0 = 0;  // S: the counts the run from zero started with
+  uint32_t blocks0 = 0, skipped0 = 0;  // S: the counts and the shift estimate the run from
+  double shift0 = 0.0;                 // zero started with
   float stripe = 0.0f;  // T: of a sample that ends escaped
   auto finish = [&](uint32_t idx, const Result &r, uint64_t nblocks, uint64_t nskipped, double sh) {
     put<B, T, L && !B && !T>(p, idx, r, T && r.kind == 0 ? stripe : 0.0f);
@@ -1515,6 +1516,7 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(Pa
     bias -= (int64_t)p.max_iter;
     blocks0 = s.blocks;
     skipped0 = s.skipped;
+    shift0 = s.shift;
     start_sample<EXT, D, L, B>(p, s, false, true);
     if (T) {  // grid.rs:638
       tr->begin();
@@ -1551,6 +1553,7 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(Pa
             if (S) {
               bias = p.series_n;
               blocks0 = skipped0 = 0;
+              shift0 = 0.0;
             }
             if (T) {  // Job::one (grid.rs:630) and the loop's start (sample.rs:235)
               tr->begin();
@@ -1598,6 +1601,7 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(Pa
         if (S) {
           s.blocks = blocks0;
           s.skipped = skipped0;
+          s.shift = shift0;
         }
         if (T) {
           tr->begin();
