@@ -958,6 +958,7 @@ __device__ __forceinline__ bool settle(const Params &p, State<EXT> &s, Result &r
   const bool limit = s.n >= s.lim;
   bool event = wild | (B && reb);
   event |= limit && (s.n == s.gate || s.n >= end || (!EXT && s.hold > 0) || (T && s.replaying));
+  event |= T && s.n >= end;  // a replay's limit may lie before lim, the block budget's
   event |= (reb && !EXT ? f2 : delta2) > RES2 * f2 && fabs(fr - s.sr) + fabs(fi - s.si) < s.near;
   if (event) {
     if (sequence<EXT, D, L, B, T>(p, s, res, make_double2(s.Zr, s.Zi), pr, pi, fr, fi, f2, product, tr)) return true;
