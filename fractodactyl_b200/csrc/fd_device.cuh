@@ -183,8 +183,9 @@ struct Contraction {
 // Every factor and product rounds within 4 units, Contraction's within 5 (normwise,
 // squared), so the two differ by less than 9 u a step. small() answers outside a band of
 // 32 u (nucleus + 8) around 1e-6 and returns -1 inside it, or where the product was lost (a
-// zero or non-finite factor, or a count beyond e's range): the sample is then iterated
-// again from its start with Contraction itself (exact()).
+// zero factor, one with a part that is not finite, one below 2^-1023, which Contraction scales
+// by an infinity into a NaN, or a count beyond e's range): the sample is then iterated again
+// from its start with Contraction itself (exact()).
 #ifndef FDK_CONTRACTION_AGAIN
 #define FDK_CONTRACTION_AGAIN false  // a test build answers -1 always
 #endif
@@ -221,7 +222,7 @@ struct Magnitude {
     r = r * f;
     i = i * f;
     const double q = r * r + i * i;
-    if (a > 0.0 && isfinite(a) && p > 0.0) {
+    if (a >= 0x1p-1023 && isfinite(q) && p > 0.0) {
       e += exponent(p) + exponent(q) - 2 * up;
       p = mantissa(p) * mantissa(q);
     } else {
