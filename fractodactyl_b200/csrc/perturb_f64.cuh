@@ -112,6 +112,7 @@ struct Params {
 
 constexpr double SAFE = 1.0 + 8.0 * U;  // sample.rs:56
 constexpr uint32_t NO_GATE = 0xffffffffu;
+constexpr int MAX_RETURNS = 4;  // near returns the extended tier counts a sample (sample.rs:494)
 
 enum : uint32_t { F_DERIV = 1u, F_BLA = 2u, F_SHIFT = 4u };
 
@@ -849,7 +850,7 @@ __device__ __forceinline__ bool sequence(const Params &p, State<EXT> &s, Result 
   if (replaying) return false;  // sample.rs:470-472: the replay only re-walks iterates
   double check_r = EXT ? pr : s.xr, check_i = EXT ? pi : s.xi;
   bool judge = check_r * check_r + check_i * check_i > RES2 * f2;
-  if (EXT) judge = judge && s.returns < 4;
+  if (EXT) judge = judge && s.returns < MAX_RETURNS;
   if (!judge) {
     if (EXT) {
       if (s.n >= s.chk) {
@@ -873,7 +874,7 @@ __device__ __forceinline__ bool sequence(const Params &p, State<EXT> &s, Result 
   }
   const double dist = fabs(fr - s.sr) + fabs(fi - s.si), near = near_bound(s);
   if (EXT) {
-    if (s.returns < 4 && dist < near) {
+    if (s.returns < MAX_RETURNS && dist < near) {
       if (contracting(p.orbit, p.last, s.m, check_r, check_i, s.ar * exp2i(s.offset_exp),
                       s.ai * exp2i(s.offset_exp), (uint64_t)(s.n - s.sn))) {
         res.kind = 2;
@@ -959,7 +960,11 @@ __device__ __forceinline__ bool settle(const Params &p, State<EXT> &s, Result &r
   bool event = wild | (B && reb);
   event |= limit && (s.n == s.gate || s.n >= end || (!EXT && s.hold > 0) || (T && s.replaying));
   event |= T && s.n >= end;  // a replay's limit may lie before lim, the block budget's
-  event |= (reb && !EXT ? f2 : delta2) > RES2 * f2 && fabs(fr - s.sr) + fabs(fi - s.si) < s.near;
+  // (a sample that has settled on a cycle stays near its save point after the last return that
+  // counts: without the test of returns 69% of the iterations of a 2.5-wide scaled-tier view
+  // without a table ran the full sequence for nothing, a batch of its frames 286 against 195 ms)
+  event |= (reb && !EXT ? f2 : delta2) > RES2 * f2 && (!EXT || s.returns < MAX_RETURNS) &&
+           fabs(fr - s.sr) + fabs(fi - s.si) < s.near;
   if (event) {
     if (sequence<EXT, D, L, B, T>(p, s, res, make_double2(s.Zr, s.Zi), pr, pi, fr, fi, f2, product, tr)) return true;
     if (s.n >= end) {  // the loop's end (sample.rs:237)
