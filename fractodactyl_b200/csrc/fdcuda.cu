@@ -1203,9 +1203,9 @@ fdc_status render_impl(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, const fdc
       ctx->blocks_per_sm[variant] = b > 0 ? b : 1;
     }
     dim3 grid(grid_blocks(ctx, ctx->blocks_per_sm[variant])), block(128);
-    const size_t trace_bytes = stripe ? sizeof(fdk::StripeTrace) * grid.x * block.x : 0;
+    const size_t trace_bytes = stripe ? sizeof(double2) * fdk::StripeTrace::UNITS * grid.x * block.x : 0;
     if (stripe) {
-      p.stripe_traces = (fdk::StripeTrace *)pool_get(ctx, trace_bytes);
+      p.stripe_traces = (double2 *)pool_get(ctx, trace_bytes);
       if (!p.stripe_traces) return fail(ctx, FDC_DEVICE_ERROR, "device memory for the stripe recorders");
     }
     // back to the pool in stream order: its next user runs after this kernel

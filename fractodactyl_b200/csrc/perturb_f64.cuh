@@ -36,8 +36,6 @@ struct Counters {
   unsigned long long pad;
 };
 
-struct StripeTrace;
-
 // Everything one launch needs; passed by value (kernel parameter space).
 struct Params {
   const double2 *__restrict__ orbit;  // Z_0..Z_last, interleaved re/im
@@ -107,7 +105,7 @@ struct Params {
   float *stripe_out;
   uint32_t stripe_window;
   double stripe_freq;
-  StripeTrace *stripe_traces;  // a recorder for every thread of the grid
+  double2 *stripe_traces;  // StripeTrace::UNITS for every thread of the grid
 };
 
 constexpr double SAFE = 1.0 + 8.0 * U;  // sample.rs:56
@@ -161,36 +159,50 @@ struct StripeSnap {
   double xr, xi;
   int32_t delta_exp;
   double scale, dc_r, dc_i;
-  uint64_t valid;  // first iterate of the recorded run that reached n
 };
 
 // The Stripe column's recorder for one lane (stripe.rs:12-241): the last 128 iterates, the
 // last 8 block starts, and the escape the blocks found while a replay re-walks its window.
-// Only the stripe variants (T) hold one. It lies in one piece in global memory (2.6 KB a lane,
-// 200 MB a grid): the iterates a lane records one after the other fill whole sectors. In local
-// memory, which interleaves a warp's lanes word by word, lanes at different iterates wrote
-// four sectors an iterate with four bytes each.
+// Only the stripe variants (T) hold one. Its 164 units of 16 bytes (2.6 KB) lie in global memory
+// in groups of 4, a warp's lanes side by side group by group: a lane that steps alone fills
+// whole sectors, lanes that step together whole lines, and a frame of short samples touches
+// few lines of what does not fit into L2. Kernel ms by units a group, 1 2 4 8 and a lane's units
+// in one piece: 1531x429 at 5e-326, 197 iterations, 0.28 0.36 0.45 0.62 1.23 (0.53 in local
+// memory, whose words are interleaved); 640x360 at 1e-100, Fixed tier, 11.6 10.7 10.4 10.5 10.5
+// (22.2); 1600x900 of the same 38.9 31.9 30.3 29.5 29.0 (99).
 struct StripeTrace {
-  static constexpr uint32_t RING = 128, SNAPS = 8;
-  double2 ring[RING];
-  StripeSnap snaps[SNAPS];
-  Result first;
-  double first_r, first_i;
-  uint64_t first_at;
+  static constexpr uint32_t RING = 128, SNAPS = 8, SNAP_UNITS = 4, FIRST = RING + SNAPS * SNAP_UNITS, UNITS = FIRST + 4,
+                            GROUP = 4;
+#if defined(__CUDA_ARCH__)
+  static constexpr uint32_t LANES = 32;
+#else
+  static constexpr uint32_t LANES = 1;  // host builds run a warp of one lane
+#endif
+  double2 *at;  // unit 0; the lanes' groups of unit 0 to 3 follow one another
   uint64_t valid;
   uint32_t count;
-  uint64_t end_at;  // the iterate the outcome's window ends at (end), and z there
+  uint32_t starts[SNAPS];  // the block starts' iterates
+  uint64_t end_at;         // the iterate the outcome's window ends at (end), and z there
   double end_r, end_i;
+
+  static __device__ __forceinline__ uint32_t place(uint32_t u) { return u / GROUP * (GROUP * LANES) + u % GROUP; }
+  __device__ __forceinline__ double2 &unit(uint32_t u) const { return at[place(u)]; }
+  static __device__ __forceinline__ double bits(uint64_t v) { return __longlong_as_double((long long)v); }
+  static __device__ __forceinline__ uint64_t bits(double v) { return (uint64_t)__double_as_longlong(v); }
 
   __device__ __forceinline__ void begin() {  // stripe.rs:164-168
     valid = ~0ull;
     count = 0;
   }
   __device__ __forceinline__ void start(uint64_t n) { valid = n + 1; }
-  __device__ __forceinline__ void record(uint64_t n, double zr, double zi) { ring[n % RING] = make_double2(zr, zi); }
-  __device__ __forceinline__ void snap(StripeSnap s, uint64_t landed) {  // stripe.rs:180-187
-    s.valid = valid;
-    snaps[count % SNAPS] = s;
+  __device__ __forceinline__ void record(uint32_t n, double zr, double zi) { unit(n % RING) = make_double2(zr, zi); }
+  __device__ __forceinline__ void snap(const StripeSnap &s, uint64_t landed) {  // stripe.rs:180-187
+    const uint32_t k = count % SNAPS, u = RING + k * SNAP_UNITS;
+    unit(u) = make_double2(bits((uint64_t)s.n << 32 | s.m), s.xr);
+    unit(u + 1) = make_double2(s.xi, bits((uint64_t)(uint32_t)s.delta_exp));
+    unit(u + 2) = make_double2(s.scale, s.dc_r);
+    unit(u + 3) = make_double2(s.dc_i, bits(valid));
+    starts[k] = s.n;
     count += 1;
     valid = landed;
   }
@@ -203,17 +215,44 @@ struct StripeTrace {
     int pick = -1;
     for (uint32_t j = 0; j < kept && pick < 0; ++j) {
       const uint32_t k = (count - 1 - j) % SNAPS;
-      if (snaps[k].n <= need) pick = (int)k;
+      if (starts[k] <= need) pick = (int)k;
     }
     if (pick < 0) {
       for (uint32_t j = 0; j < kept; ++j) {
         const uint32_t k = (count - 1 - j) % SNAPS;
-        if (pick < 0 || snaps[k].n < snaps[pick].n) pick = (int)k;
+        if (pick < 0 || starts[k] < starts[pick]) pick = (int)k;
       }
     }
-    valid = snaps[pick].valid;
-    out = snaps[pick];
+    const uint32_t u = RING + (uint32_t)pick * SNAP_UNITS;
+    const double2 a = unit(u), b = unit(u + 1), c = unit(u + 2), d = unit(u + 3);
+    out.m = (uint32_t)bits(a.x);
+    out.n = (uint32_t)(bits(a.x) >> 32);
+    out.xr = a.y;
+    out.xi = b.x;
+    out.delta_exp = (int32_t)(uint32_t)bits(b.y);
+    out.scale = c.x;
+    out.dc_r = c.y;
+    out.dc_i = d.x;
+    valid = bits(d.y);
     return true;
+  }
+  // the escape the blocks found, kept while a replay re-walks its window
+  __device__ __forceinline__ void keep(const Result &r) {
+    unit(FIRST) = make_double2(bits(r.n), bits((uint64_t)r.dexp));
+    unit(FIRST + 1) = make_double2(r.zr, r.zi);
+    unit(FIRST + 2) = make_double2(r.dr, r.di);
+  }
+  __device__ __forceinline__ Result kept() const {
+    const double2 a = unit(FIRST), z = unit(FIRST + 1), d = unit(FIRST + 2);
+    Result r;
+    r.kind = 0;
+    r.n = bits(a.x);
+    r.dexp = (int64_t)bits(a.y);
+    r.zr = z.x;
+    r.zi = z.y;
+    r.dr = d.x;
+    r.di = d.y;
+    return r;
   }
   // stripe.rs:132-152: 0.5 + 0.5 sin(k arg z); a whole k up to 16 as the sign of k times
   // Im (z / |z|)^|k|
@@ -241,16 +280,13 @@ struct StripeTrace {
     end_i = zi;
   }
   // stripe.rs:206-240: the windows ending at z_n and z_{n-1}, interpolated by how far past the
-  // escape radius z_n landed, by a whole warp: each lane takes the term of one iterate, and
-  // all add them in the reference's order. One lane after the other for every finished
-  // sample, the terms (a hypot, two divisions or a sine each) were most of the kernel's work.
-  __device__ float average(unsigned lane, double r2, uint32_t window, double k) const {
-#if defined(__CUDA_ARCH__)
-    constexpr uint64_t LANES = 32;
-#else
-    constexpr uint64_t LANES = 1;  // host builds run a warp of one lane
-#endif
-    const uint64_t n = end_at, from = valid;
+  // escape radius z_n landed, of lane l's sample by the whole warp: each lane takes the term of one
+  // iterate, and all add them in the reference's order. One lane after the other for every
+  // finished sample, the terms (a hypot, two divisions or a sine each) were most of the kernel's
+  // work. The value is lane l's; the others' is of no use.
+  __device__ float average(unsigned lane, unsigned l, double r2, uint32_t window, double k) const {
+    const uint64_t n = __shfl_sync(0xffffffffu, end_at, (int)l), from = __shfl_sync(0xffffffffu, valid, (int)l);
+    const double2 *ring = at + ((int)l - (int)lane) * (int)GROUP;
     const uint64_t lo = n > window ? n - window : 0;
     const uint64_t first_i = lo > 1 ? lo : 1;
     double now = 0.0, before = 0.0;
@@ -259,7 +295,7 @@ struct StripeTrace {
       const uint64_t mine = base + lane;
       double own = 0.0;
       if (mine <= n && mine >= from) {
-        const double2 z = ring[mine % RING];
+        const double2 z = ring[place((uint32_t)(mine % RING))];
         own = term(z.x, z.y, k);
       }
       for (uint64_t i = base; i < base + LANES && i <= n; ++i) {
@@ -714,15 +750,12 @@ __device__ __forceinline__ bool sequence(const Params &p, State<EXT> &s, Result 
     if (T) {  // sample.rs:387-403
       if (replaying) {  // the replay reached an escape: the blocks' outcome, this window
         tr->end(s.n, fr, fi);
-        res = tr->first;
+        res = tr->kept();
         return true;
       }
       StripeSnap sn;
       if (tr->rewind(s.n, p.stripe_window, sn)) {
-        tr->first = res;
-        tr->first_at = s.n;
-        tr->first_r = fr;
-        tr->first_i = fi;
+        tr->keep(res);
         s.replaying = true;
         const uint64_t give_up = (uint64_t)s.n + 64;  // sample.rs:397
         s.limit = (uint32_t)(give_up < p.max_iter ? give_up : p.max_iter);
@@ -969,8 +1002,8 @@ __device__ __forceinline__ bool settle(const Params &p, State<EXT> &s, Result &r
     if (sequence<EXT, D, L, B, T>(p, s, res, make_double2(s.Zr, s.Zi), pr, pi, fr, fi, f2, product, tr)) return true;
     if (s.n >= end) {  // the loop's end (sample.rs:237)
       if (T && s.replaying) {  // sample.rs:576-579: the replay gave up; from what was recorded
-        tr->end(tr->first_at, tr->first_r, tr->first_i);
-        res = tr->first;
+        res = tr->kept();
+        tr->end(res.n, res.zr, res.zi);
       } else {
         res.kind = 2;
       }
@@ -1167,7 +1200,7 @@ __device__ __forceinline__ unsigned warp_step(const Params &p, State<EXT> &s, Re
       uint32_t at;
       const int lv = block_level<EXT, T>(p, s, at);
       if (T)  // sample.rs:267-281: the block start, for a later replay
-        tr->snap(StripeSnap{s.m, s.n, s.xr, s.xi, s.delta_exp, s.scale, s.dc_r, s.dc_i, 0}, s.n + (2u << lv));
+        tr->snap(StripeSnap{s.m, s.n, s.xr, s.xi, s.delta_exp, s.scale, s.dc_r, s.dc_i}, s.n + (2u << lv));
       apply_block<EXT, D>(p, s, lv, at, product);
       upd = true;
     }
@@ -1462,14 +1495,21 @@ struct TraceSlot {
 };
 template <>
 struct TraceSlot<true> {
-#if defined(__CUDA_ARCH__)
-  __device__ __forceinline__ StripeTrace *get(const Params &p) {
-    return p.stripe_traces + ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
-  }
-#else
-  StripeTrace t;  // host builds of this header
-  StripeTrace *get(const Params &) { return &t; }
+  StripeTrace t;
+#if !defined(__CUDA_ARCH__)
+  double2 units[StripeTrace::UNITS];  // host builds of this header
 #endif
+  __device__ __forceinline__ StripeTrace *get(const Params &p) {
+#if defined(__CUDA_ARCH__)
+    const size_t thread = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    t.at = p.stripe_traces + (thread / 32 * StripeTrace::UNITS * 32 + thread % 32 * StripeTrace::GROUP);
+#else
+    t.at = units;
+#endif
+    t.begin();
+    t.end(0, 0.0, 0.0);
+    return &t;
+  }
 };
 
 // The BLA variants outside B and T store finished samples' raw state only (put's R: every
@@ -1594,7 +1634,7 @@ __global__ void __launch_bounds__(128, Occupancy<EXT>::blocks) perturb_kernel(Pa
       while (todo) {
         const unsigned l = (unsigned)__ffs((int)todo) - 1u;
         todo &= todo - 1u;
-        const float v = (tr + ((int)l - (int)lane))->average(lane, p.r2, p.stripe_window, p.stripe_freq);
+        const float v = tr->average(lane, l, p.r2, p.stripe_window, p.stripe_freq);
         if (l == lane) stripe = v;
       }
     }

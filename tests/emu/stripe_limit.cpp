@@ -33,14 +33,14 @@ static uint32_t replay(uint32_t limit, uint32_t lim) {
   s.ai = 0.02;
   s.offset_exp = 0;
   fdk::start_sample<EXT, D, true, false>(p, s, false, false);
-  fdk::StripeTrace tr;
-  tr.begin();
+  fdk::TraceSlot<true> slot;
+  fdk::StripeTrace &tr = *slot.get(p);
   tr.start(0);
-  tr.first = fdk::Result{};
-  tr.first.n = 77;
-  tr.first_at = 77;
-  tr.first_r = 3.0;
-  tr.first_i = 4.0;
+  fdk::Result first{};
+  first.n = 77;
+  first.zr = 3.0;
+  first.zi = 4.0;
+  tr.keep(first);
   s.replaying = true;
   s.limit = limit;
   s.lim = lim;
