@@ -13,7 +13,7 @@ LIB_PATH = os.path.join(HERE, "libfdcuda.so")
 OK, DECLINED, INVALID, DEVICE_ERROR, TIMEOUT, NO_DEVICE = range(6)
 STATUS_NAMES = {0: "OK", 1: "DECLINED", 2: "INVALID", 3: "DEVICE_ERROR", 4: "TIMEOUT", 5: "NO_DEVICE"}
 # fdc_job flags
-DERIVATIVE, BLA, SHIFT, F32, DEVICE_OUT, SERIES = 1, 2, 4, 8, 16, 32
+DERIVATIVE, BLA, SHIFT, F32, DEVICE_OUT, SERIES, BAND = 1, 2, 4, 8, 16, 32, 64
 
 
 class Job(C.Structure):

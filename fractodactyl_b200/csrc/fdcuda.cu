@@ -21,6 +21,7 @@
 
 #include "../../include/fdcuda.h"
 #include "launch.hpp"
+#include "launch_shape.hpp"
 #include "bla_build.cuh"
 #include "perturb_f64.cuh"
 #include "route_internal.hpp"
@@ -1173,21 +1174,16 @@ fdc_status render_impl(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, const fdc
   p.timed_out = &ctx->scratch->timed_out;
   CK(cudaMemsetAsync(ctx->scratch, 0, sizeof(Scratch), ctx->stream));
 
-  const uint64_t resident = ext && !(j.flags & FDC_F32) ? fdk::Occupancy<true>::blocks : fdk::Occupancy<false>::blocks;
-  // A launch of few samples spreads them over 12 warps an SM instead of filling the first
-  // warps: a warp of 32 lanes that diverge runs every lane's branches and waits for every
-  // lane's table loads (kernel ms at full warps / 4, 8, 12, 16 warps an SM: 64x36 shallow
-  // 0.418 / 0.343 0.333 0.329 0.351, 161x91 with blocks 1.12 / 1.09 0.95 0.85 0.94).
-  // Over the last three waves of the grid a warp reserves no slots ahead (401x227 without a
-  // table 1.15 -> 0.86 ms, 480x270 2.72 -> 2.49; an eighth of the queue where that is more).
-  const uint64_t spread = (uint64_t)ctx->sm_count * 12, lanes = (p.total + spread - 1) / spread;
-  p.idle_lanes = lanes < 32 ? (uint32_t)(32 - lanes) : 0;
-  p.tail = (uint32_t)std::max<uint64_t>(p.total / 8, 3ull * ctx->sm_count * resident * 128);
+  uint64_t frame_slots = p.total;  // of the frame that a band stands for
+  if (j.flags & FDC_BAND) {
+    const uint64_t tw = 1ull << p.tile_shift, th = 32ull >> p.tile_shift;
+    frame_slots = (j.nx + tw - 1) / tw * ((j.ny + th - 1) / th) * 32;
+  }
 
   uint32_t launches = 1;
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   if (j.flags & FDC_F32) {
-    CK(fdk::launch_f32(p, o.z32, deriv, bla, ctx->sm_count, (int)ctx->tune.blocks_per_sm, ctx->stream,
+    CK(fdk::launch_f32(p, frame_slots, o.z32, deriv, bla, ctx->sm_count, (int)ctx->tune.blocks_per_sm, ctx->stream,
                        ctx->blocks_per_sm_f32));
     if (encode_later && (p.nu || p.de || p.normal)) {
       fdk::encode_kernel<0><<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(p);
@@ -1203,6 +1199,12 @@ fdc_status render_impl(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, const fdc
       ctx->blocks_per_sm[variant] = b > 0 ? b : 1;
     }
     dim3 grid(grid_blocks(ctx, ctx->blocks_per_sm[variant])), block(128);
+    const fdk::LaunchShape shape =
+        fdk::launch_shape(p.total, frame_slots, ctx->sm_count, grid.x / ctx->sm_count,
+                          ext ? fdk::Occupancy<true>::blocks : fdk::Occupancy<false>::blocks,
+                          ext && !bla ? fdk::SPREAD_WARPS_EXT_PLAIN : fdk::SPREAD_WARPS);
+    p.idle_lanes = shape.idle_lanes;
+    p.tail = shape.tail;
     const size_t trace_bytes = stripe ? sizeof(double2) * fdk::StripeTrace::UNITS * grid.x * block.x : 0;
     if (stripe) {
       p.stripe_traces = (double2 *)pool_get(ctx, trace_bytes);

@@ -111,7 +111,7 @@ class Tuner:
                 C.memmove(C.byref(j), C.byref(job), C.sizeof(_lib.Job))
                 j.first_row, j.rows = first, rows
                 j.flags = (job.flags | _lib.F32) if s.f32 else (job.flags & ~_lib.F32)
-                j.flags &= ~_lib.DEVICE_OUT
+                j.flags = (j.flags & ~_lib.DEVICE_OUT) | _lib.BAND  # the launch whose settings are sought
                 best = float("inf")
                 for _ in range(self.reps):
                     arrays, cnt, _ = self.dev.render_job(j, columns=())

@@ -45,7 +45,10 @@ enum {
   FDC_SHIFT = 1u << 2,      /* accumulate the BLA first-order shift estimate (BlaStats.shift_px) */
   FDC_F32 = 1u << 3,        /* precision form: FP32-mantissa floatexp deltas (not bit-exact) */
   FDC_DEVICE_OUT = 1u << 4, /* fdc_out pointers are device pointers (no host copies) */
-  FDC_SERIES = 1u << 5      /* start every sample from the orbit's uploaded series */
+  FDC_SERIES = 1u << 5,     /* start every sample from the orbit's uploaded series */
+  FDC_BAND = 1u << 6        /* the rows stand for the whole frame: launched as its render would be
+                             * (a launch of few samples takes another shape); results do not
+                             * depend on it. For measuring launch settings on part of a frame. */
 };
 
 typedef struct fdc_ctx fdc_ctx;
