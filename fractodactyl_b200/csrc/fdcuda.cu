@@ -98,6 +98,9 @@ struct fdc_ctx {
   // next upload of the same size: a film or a service re-uploading per frame allocates
   // once. Stream-ordered: every user runs on `stream`. Freed by fdc_close.
   std::multimap<size_t, void *> pool;
+  // stripe recorders: one buffer for the largest stripe launch so far. Freed by fdc_close.
+  double2 *traces = nullptr;
+  size_t trace_bytes = 0;
   char *small = nullptr;  // pinned staging of a small render's columns and counters
   // pinned staging for large host<->device copies: two chunk slots, each with the event
   // of the last transfer that used it
@@ -762,6 +765,7 @@ void fdc_close(fdc_ctx *ctx) {
     if (ev) cudaEventDestroy(ev);
   cudaFree(ctx->scratch);
   cudaFree(ctx->stage);
+  cudaFree(ctx->traces);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -1205,13 +1209,23 @@ fdc_status render_impl(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, const fdc
                           ext && !bla ? fdk::SPREAD_WARPS_EXT_PLAIN : fdk::SPREAD_WARPS);
     p.idle_lanes = shape.idle_lanes;
     p.tail = shape.tail;
-    const size_t trace_bytes = stripe ? sizeof(double2) * fdk::StripeTrace::UNITS * grid.x * block.x : 0;
-    if (stripe) {
-      p.stripe_traces = (double2 *)pool_get(ctx, trace_bytes);
-      if (!p.stripe_traces) return fail(ctx, FDC_DEVICE_ERROR, "device memory for the stripe recorders");
+    if (stripe) {  // a recorder for every thread, so no more blocks than have samples to take
+      const uint64_t takes = 4 * (32 - p.idle_lanes);
+      grid.x = (unsigned)std::min<uint64_t>(grid.x, (p.total + takes - 1) / takes);
+      const size_t bytes = sizeof(double2) * fdk::StripeTrace::UNITS * grid.x * block.x;
+      if (bytes > ctx->trace_bytes) {
+        CK(cudaStreamSynchronize(ctx->stream));
+        cudaFree(ctx->traces);
+        ctx->traces = nullptr;
+        ctx->trace_bytes = 0;
+        if (cudaMalloc(&ctx->traces, bytes) != cudaSuccess) {
+          cudaGetLastError();  // the failure is reported here
+          return fail(ctx, FDC_DEVICE_ERROR, "device memory for the stripe recorders");
+        }
+        ctx->trace_bytes = bytes;
+      }
+      p.stripe_traces = ctx->traces;
     }
-    // back to the pool in stream order: its next user runs after this kernel
-    pool_put(ctx, p.stripe_traces, trace_bytes);
     void *args[] = {&p};
     CK(cudaLaunchKernel(fn, grid, block, args, 0, ctx->stream));
     CK(cudaGetLastError());

@@ -175,8 +175,9 @@ fdc_status fdc_render_bounded(fdc_ctx *ctx, const fdc_job *job, fdc_out *out, co
  * layout, FDC_DEVICE_OUT included); the average's terms use CUDA's hypot / sin / atan2 /
  * log, so values are within a few ulps of the CPU's. FDC_INVALID: window outside 1..64 or
  * a frequency that is not finite. FDC_DECLINED (render on the CPU): FDC_SERIES, FDC_F32.
- * Each resident lane's recorder (2.6 KB, 200 MB in all) is device memory of the context,
- * kept for the next such render and given back by fdc_close. */
+ * Each thread of the launch has a recorder of 2.6 KB in device memory of the context: one buffer
+ * for the largest such launch so far (up to 199 MB on the ordinary tiers, 249 MB on the scaled
+ * one, on 148 SMs; less for frames of few samples), given back by fdc_close. */
 typedef struct {
   uint32_t window; /* iterates averaged before escape, 1..64 (StripeParams, stripe.rs:20-36) */
   double freq;     /* k of 0.5 + 0.5 sin(k arg z) */
