@@ -312,22 +312,20 @@ LevelTable level_table(const BlaDev &d) {
   return t;
 }
 
-// The fused stream: point m with the squared radii of the level-0 and level-1 blocks
-// starting at Z_m (block t of level i starts at m = 1 + t 2^(i+1), bla.rs:131-135), -1
-// where none starts; the level-0 radius also goes into the precision-form entries.
-__global__ void fuse_bla(const double2 *__restrict__ z, uint64_t len, const double *__restrict__ r2, uint32_t levels,
-                         uint64_t off0, uint64_t cnt0, uint64_t off1, uint64_t cnt1, double *__restrict__ fused,
-                         double *__restrict__ z32) {
+// The fused stream: point m with the squared radius of the level-0 block starting at Z_m
+// (block t of level i starts at m = 1 + t 2^(i+1), bla.rs:131-135), -1 where none starts, in
+// 32 bytes; the radius also goes into the precision-form entries.
+__global__ void fuse_bla(const double2 *__restrict__ z, uint64_t len, const double *__restrict__ r2, uint64_t blocks,
+                         double *__restrict__ fused, double *__restrict__ z32) {
   for (uint64_t m = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; m < len; m += (uint64_t)gridDim.x * blockDim.x) {
     const double2 p = z[m];
-    double a = -1.0, b = -1.0;
-    if (m >= 1 && levels > 0 && ((m - 1) & 1) == 0 && ((m - 1) >> 1) < cnt0) a = r2[off0 + ((m - 1) >> 1)];
-    if (m >= 1 && levels > 1 && ((m - 1) & 3) == 0 && ((m - 1) >> 2) < cnt1) b = r2[off1 + ((m - 1) >> 2)];
+    double a = -1.0;
+    if (m >= 1 && ((m - 1) & 1) == 0 && ((m - 1) >> 1) < blocks) a = r2[(m - 1) >> 1];
     double *f = fused + 4 * m;
     f[0] = p.x;
     f[1] = p.y;
     f[2] = a;
-    f[3] = b;
+    f[3] = 0.0;
     z32[4 * m + 3] = a;
   }
 }
@@ -884,9 +882,7 @@ fdc_status fdc_upload_bla(fdc_ctx *ctx, int32_t orbit, const double *blocks7, co
     return fail(ctx, FDC_INVALID, (flags & 1) ? "BLA level holds a non-finite value"
                                               : "BLA level holds a negative radius");
   }
-  fuse_bla<<<grid_for(o.len), 256, 0, ctx->stream>>>(o.z, o.len, d.r2, levels, levels > 0 ? d.off[0] : 0,
-                                                     levels > 0 ? d.count[0] : 0, levels > 1 ? d.off[1] : 0,
-                                                     levels > 1 ? d.count[1] : 0, d.fused, o.z32);
+  fuse_bla<<<grid_for(o.len), 256, 0, ctx->stream>>>(o.z, o.len, d.r2, levels > 0 ? d.count[0] : 0, d.fused, o.z32);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     free_bla(ctx, d);
@@ -986,9 +982,7 @@ fdc_status fdc_build_bla(fdc_ctx *ctx, int32_t orbit, double eps, double dc_max,
     return fail(ctx, FDC_INVALID, (badf & 1) ? "BLA level holds a non-finite value"
                                              : "BLA level holds a negative radius");
   }
-  fuse_bla<<<grid_for(o.len), 256, 0, ctx->stream>>>(o.z, o.len, d.r2, kept, kept > 0 ? d.off[0] : 0,
-                                                     kept > 0 ? d.count[0] : 0, kept > 1 ? d.off[1] : 0,
-                                                     kept > 1 ? d.count[1] : 0, d.fused, o.z32);
+  fuse_bla<<<grid_for(o.len), 256, 0, ctx->stream>>>(o.z, o.len, d.r2, kept > 0 ? d.count[0] : 0, d.fused, o.z32);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     free_bla(ctx, d);

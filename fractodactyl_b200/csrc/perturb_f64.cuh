@@ -39,9 +39,9 @@ struct Counters {
 // Everything one launch needs; passed by value (kernel parameter space).
 struct Params {
   const double2 *__restrict__ orbit;  // Z_0..Z_last, interleaved re/im
-  // With BLA: Z_m fused with the squared radii of the level-1 and level-2 blocks (j = 1, 2)
-  // starting at m, or -1 where none starts there: 32-byte entries (zr, zi, r2a, r2b), one load
-  // each, so that whether a block starts comes with the orbit point each step loads anyway.
+  // With BLA: Z_m fused with the squared radius of the first-level block (2 steps) starting at m,
+  // -1 where none starts there: 32-byte entries (zr, zi, r2a, unused), one load each, so that
+  // whether a block starts comes with the orbit point each step loads anyway.
   const double2 *__restrict__ fused;
   const void *orbit32;  // precision-form entries (perturb_f32.cuh), per job in batches
   uint32_t last;
@@ -486,7 +486,7 @@ __device__ __forceinline__ Block4 load_block(const double2 *at) {
 }
 
 // The orbit entry at m: Z_m, and with BLA the squared radius of the first-level block there,
-// in one 32-byte load (its fourth value, the second level's radius, is read by block_level).
+// in one 32-byte load, whose fourth value is unused.
 struct Entry {
   double zr, zi, r2a;
 };
@@ -496,9 +496,9 @@ __device__ __forceinline__ Entry load_entry(const Params &p, uint32_t m) {
   if (L) {
 #if defined(__CUDA_ARCH__)
     Entry e;
-    double r2b;
+    double unused;
     asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-        : "=d"(e.zr), "=d"(e.zi), "=d"(e.r2a), "=d"(r2b)
+        : "=d"(e.zr), "=d"(e.zi), "=d"(e.r2a), "=d"(unused)
         : "l"(p.fused + 2 * m));
     return e;
 #else
