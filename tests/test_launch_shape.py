@@ -74,9 +74,13 @@ def test_tuner_measures_bands_as_the_frame():
             cnt = _lib.Counters(kernel_ms=1.0)
             return {"cls": np.zeros(n, np.uint8), "n": np.zeros(n, np.uint32)}, cnt, 0
 
-    job = _lib.Job(nx=64, ny=128, flags=_lib.DERIVATIVE | _lib.DEVICE_OUT)
-    tuner = tune.Tuner(Dev(), settings=[tune.Setting(4), tune.Setting(8)], reps=1)
-    tuner.choice(job)
-    assert len(flags) == 3 * len(tune.bands(128))
-    assert all(f & _lib.BAND and not f & _lib.DEVICE_OUT for f, _, _ in flags)
-    assert job.flags == _lib.DERIVATIVE | _lib.DEVICE_OUT
+    for nx, ny, launches in ((64, 128, 1), (1920, 1080, 1), (1920, 1200, 2)):
+        flags.clear()
+        job = _lib.Job(nx=nx, ny=ny, flags=_lib.DERIVATIVE | _lib.DEVICE_OUT)
+        tune.Tuner(Dev(), settings=[tune.Setting(4), tune.Setting(8)], reps=1).choice(job)
+        assert len(flags) == 3 * launches
+        assert all(f & _lib.BAND and not f & _lib.DEVICE_OUT for f, _, _ in flags)
+        assert job.flags == _lib.DERIVATIVE | _lib.DEVICE_OUT
+        rows = sum(r for _, _, r in flags[:launches])
+        assert rows == ny if launches == 1 else abs(rows * nx - (1 << 20)) <= 4 * nx
+        assert all(0 <= f and f + r <= ny for _, f, r in flags)
