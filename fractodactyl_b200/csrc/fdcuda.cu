@@ -111,14 +111,12 @@ struct fdc_ctx {
   std::map<std::tuple<uint32_t, uint32_t, uint32_t>, uint32_t *> orders;
 };
 
-// Persistent grid of a plain-form kernel: the occupancy limit, or fewer blocks per SM
-// when the tuning asks for fewer.
 // Lanes a warp gathers before applying BLA blocks (fdc_tuning.defer; 0: per variant). The
 // extended tier's blocks carry renormalisations and gather more lanes. Kernel ms over 4, 6,
-// 8, 10, 12, 16: 1920x1080 at a 1e-100 nucleus, extended tier 27.2 25.6 24.3 23.6 23.3 24.1;
-// 1280x720 on the Fixed tier 11.7 12.1 12.5 12.6 13.1 14.2.
-// The precision form over 2, 3, 4, 6, 8, 12: 960x540 at 1e-100, extended tier 9.52 9.59 9.77 9.95 10.06
-// 10.48; at 1e-70 on the Fixed tier 6.04 5.93 5.90 5.74 5.73 5.76.
+// 8, 10, 12, 16: 1920x1080 at a 1e-100 nucleus, extended tier 23.2 21.6 20.5 19.9 19.7 20.5;
+// Fixed tier 1280x720 9.9 10.4 10.7 11.0 11.4 12.4, 1920x1080 19.8 at 4, 18.3 at 8. The precision
+// form over 2, 3, 4, 6, 8, 12: 960x540 at 1e-100, extended tier 9.39 9.55 9.65 9.91 10.15 10.53; at
+// 1e-70 on the Fixed tier 5.77 5.64 5.61 5.54 5.48 5.44.
 static uint32_t defer_for(const fdc_ctx *ctx, bool ext, bool f32) {
   if (ctx->tune.defer > 0) return ctx->tune.defer;
   return f32 ? (ext ? 3u : 8u) : (ext ? 12u : 4u);
@@ -153,6 +151,8 @@ static const uint32_t *centre_first(fdc_ctx *ctx, uint32_t tiles_x, uint32_t til
   return dev;
 }
 
+// Persistent grid of a plain-form kernel: the occupancy limit, or fewer blocks per SM
+// when the tuning asks for fewer.
 static int grid_blocks(const fdc_ctx *ctx, int occupancy) {
   int b = occupancy;
   if (ctx->tune.blocks_per_sm > 0 && (int)ctx->tune.blocks_per_sm < b) b = (int)ctx->tune.blocks_per_sm;
@@ -1416,8 +1416,9 @@ fdc_status fdc_batch_create(fdc_ctx *ctx, const fdc_job *jobs, const fdc_out *ou
       }
     }
   }
-  // group by kernel variant; within a group the deepest jobs first (their samples run
-  // longest, so starting them first shortens the tail of the launch)
+  // group by kernel variant; within a group the deepest jobs first: over one location's orbit
+  // (a film) their samples run longest, and starting them first shortens the tail of the
+  // launch. Between locations depth says little about length.
   std::map<int, std::vector<uint32_t>> by;
   for (uint32_t k = 0; k < njobs; ++k) by[key[k]].push_back(k);
   uint32_t base = 0;

@@ -386,8 +386,10 @@ __device__ __forceinline__ bool block_starts(const State<EXT> &s) {
 // many with 6 radii in two rounds of loads instead of 8 and more: every third level, then the
 // two between (kernel ms: 2880x1620 jittered 1e-300 51.7 -> 48.7, 1920x1080 1e-100 20.0 -> 19.5,
 // tiles batch 16.7 -> 16.0). Blocks of the 1e-100 nucleus view are 2^7 steps long in the
-// median. WIDE: levels 1-8 in one round of loads, for the stripe variants, whose recorders
-// drive the table out of L1 (640x360 10.8 against 12.0 ms).
+// median. WIDE: levels 1-8 in one round of loads, for the stripe variants:
+// a frame that ends with its longest samples gains a round's latency, a large one pays the loads
+// (Fixed tier at 1e-100, 640x360 10.4 against 10.9 ms, 1600x900 30.3 against 29.2; Scaled tier 640x360
+// 8.35 against 8.30).
 template <bool EXT, bool WIDE>
 __device__ __forceinline__ int block_level(const Params &p, const State<EXT> &s, uint32_t &at) {
   const double d2 = block_d2(s);
